@@ -2,9 +2,12 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
+#include <system_error>
 #include <vector>
 
 #include "../../include/fvdbm.h"
@@ -18,6 +21,16 @@ std::mutex g_err_mu;
 std::string g_create_err;
 
 constexpr int kGraphSteps = 32;  // steps per captured graph (even)
+// Runs of at least this many steps go to the resident kernel, when the state
+// fits on the chip: its launch loads and stores the whole state (about 20 us
+// with the launch), which a short run does not win back.  us per step, per-step
+// kernels / resident: 60k cells 13.0 / 9.9 at 4 steps, 8.2 / 3.2 at 512; 250k
+// 16.1 / 15.2 and 10.9 / 7.6; 400k 15.8 / 17.0 at 4, 13.2 / 12.4 at 8, 10.7 /
+// 7.9 at 512.  A launch takes at most kResidentSteps.
+constexpr int kResidentMin = 4, kResidentMinLarge = 8;
+constexpr int kLargeMesh = 1 << 18;  // cells from which AUTO takes the single-launch family
+constexpr int kResidentSteps = 1 << 20;
+constexpr int kResidentCells = 96;  // cells per block, at least (3.2k cells: 3.4 us per step, 3.9 at 128)
 
 struct Handle {
   int device = 0;
@@ -39,6 +52,12 @@ struct Handle {
   bool one = false;  // node and cell blocks in one launch
   bool persist = false;  // FVDBM_KERNEL_PERSIST: one cooperative launch per fvdbm_step call
   int* bar = nullptr;    // its grid-barrier counter
+  // resident step (resident.cu): runs of several steps in one launch, with the
+  // state on the chip; res_tag: exchange tags used so far
+  bool resident = false;
+  DevResident res{};
+  size_t res_ex_bytes = 0;
+  unsigned res_tag = 0;
   // packed batch of independent cases (fvdbm_batch_create)
   bool batch = false;
   int batch_block = 256, batch_waves = 1;
@@ -250,7 +269,40 @@ int ensure_nodes(Handle* h) {
 
 constexpr int kPersistSteps = 4096;  // steps per cooperative launch, at most
 
+// A resident run may be queued: not while the stream is being captured (the
+// exchange tags of a launch serve once, so it must not be replayed).
+bool resident_ready(Handle* h) {
+  if (!h->resident) return false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
+// n steps in resident launches.  Afterwards the handle is as after n single
+// steps: both pdf buffers, the nodes of the last step, the stencil macros.
+int run_resident(Handle* h, int n) {
+  while (n > 0) {
+    const int k = std::min(n, kResidentSteps);
+    if (h->res_tag > 0xffffffffu - unsigned(k)) {
+      CK(cudaMemsetAsync(h->res.ex, 0, h->res_ex_bytes, h->stream));
+      h->res_tag = 0;
+    }
+    const DevPlan p = h->fnodes ? with_nodes(h, h->node_cur, h->node_cur) : h->dp;
+    const int last = h->cur ^ (k & 1);
+    CK(launch_resident(p, h->res, h->f[h->cur], h->f[last ^ 1], h->f[last], k, h->res_tag, h->stream));
+    h->res_tag += unsigned(k);
+    h->cur = last;
+    if (h->fnodes) {
+      h->node_last = h->node_cur;
+      h->node_cur ^= 1;
+      h->nodes_ready = false;
+    }
+    n -= k;
+  }
+  return FVDBM_OK;
+}
+
 int enqueue_steps(Handle* h, int n) {
+  if (h->persist && resident_ready(h)) return run_resident(h, n);
   if (h->persist) {
     for (int done = 0; done < n;) {
       const int k = std::min(n - done, kPersistSteps);
@@ -349,6 +401,79 @@ int get_graph(Handle* h, int parity, cudaGraphExec_t* out) {
   return FVDBM_OK;
 }
 
+// Tables of the resident step, when the state of this mesh fits on the chip:
+// planned beside the rest of fvdbm_create (start), then uploaded (make).
+std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh) {
+  int sms = 0, lim = 0;
+  const HostPlan& hp = h->hp;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess || hp.N == 0 ||
+      int64_t(hp.N) * 2 * hp.q * 4 > int64_t(sms) * lim)
+    return {};
+  const int blocks = std::min(sms, (hp.N + kResidentCells - 1) / kResidentCells);
+  auto plan = [h, &mesh, blocks] {
+    ResidentPlan rp;
+    build_resident(mesh, h->params, h->hp, blocks, rp);
+    return rp;
+  };
+  try {
+    return std::async(std::launch::async, plan);
+  } catch (const std::system_error&) {  // no thread to be had: planned when it is asked for
+    return std::async(std::launch::deferred, plan);
+  }
+}
+
+int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
+  if (!plan.valid()) return FVDBM_OK;
+  const HostPlan& hp = h->hp;
+  ResidentPlan rp;
+  try {
+    rp = plan.get();
+  } catch (const std::bad_alloc&) {
+    return fail(h, FVDBM_ENOMEM, "host memory for the resident step's tables");
+  }
+  if (!rp.ok) return FVDBM_OK;
+  DevResident& r = h->res;
+  bool fits = false;
+  CK(prepare_resident(h->dp, rp, r, &fits));
+  if (!fits) return FVDBM_OK;
+  // one allocation and one copy for all tables
+  std::vector<unsigned char> buf;
+  std::vector<std::pair<const void**, size_t>> at;  // field, offset
+  auto put = [&](auto& field, const auto& vec) {
+    const size_t o = (buf.size() + 255) / 256 * 256, n = vec.size() * sizeof(vec[0]);
+    buf.resize(o + std::max<size_t>(n, 16));
+    if (n) std::memcpy(buf.data() + o, vec.data(), n);
+    at.push_back({reinterpret_cast<const void**>(&field), o});
+  };
+  put(r.block, rp.block);
+  put(r.dev, rp.dev);
+  put(r.exp, rp.exp);
+  put(r.cls, rp.cls);
+  put(r.hf, rp.hf);
+  put(r.inv_area, rp.inv_area);
+  put(r.halo_dev, rp.halo_dev);
+  put(r.halo_exp, rp.halo_exp);
+  put(r.st_loc, rp.st_loc);
+  put(r.nd, rp.nd);
+  put(r.nd_sw, rp.nd_sw);
+  put(r.en_st, rp.en_st);
+  put(r.en_w, rp.en_w);
+  put(r.fz_dev, rp.fz_dev);
+  put(r.gh, rp.gh);
+  unsigned char* base = nullptr;
+  int rc = dalloc(h, &base, buf.size(), &buf);
+  if (rc != FVDBM_OK) return rc;
+  for (auto& a : at) *a.first = base + a.second;
+  const size_t words = size_t(2) * ((hp.q + 2) / 3) * size_t(std::max(rp.n_export, 1));
+  if ((rc = dalloc<uint4>(h, &r.ex, words)) != FVDBM_OK) return rc;
+  h->res_ex_bytes = words * sizeof(uint4);
+  CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));
+  CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
+  h->resident = true;
+  return FVDBM_OK;
+}
+
 // Cell blocks (of the batch launch's block size) holding cells of active
 // cases; the launch covers only those.  The grid size changes, so captured
 // graphs are dropped.
@@ -413,7 +538,9 @@ int fvdbm_destroy(void* handle) {
 
 static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, const BatchSegs* segs,
                        const float* case_inv_tau, const float* case_dt, void** handle) {
+  std::future<ResidentPlan> resident_plan;
   auto create_fail = [&](Handle* h, int code) {
+    if (resident_plan.valid()) resident_plan.wait();  // it reads h
     {
       std::lock_guard<std::mutex> lk(g_err_mu);
       g_create_err = h ? h->err : "invalid arguments";
@@ -433,7 +560,7 @@ static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, c
   // 9.9 us at 3.2k cells, 10.0 against 11.5 us at 60k)
   const bool auto_family = params->kernel == FVDBM_KERNEL_AUTO && !segs;
   fvdbm_params_t pplan = *params;
-  if (auto_family && mesh->n_cells >= (1 << 18)) pplan.kernel = FVDBM_KERNEL_FUSED_NODES;
+  if (auto_family && mesh->n_cells >= kLargeMesh) pplan.kernel = FVDBM_KERNEL_FUSED_NODES;
   std::string why = build_plan(mesh, &pplan, h->hp, segs);
   if (!why.empty()) {
     h->err = why;
@@ -518,6 +645,8 @@ static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, c
     h->batch = true;
     h->fused = h->tile = h->one = false;
   }
+  if (h->persist || params->kernel == FVDBM_KERNEL_FAST || (auto_family && (h->fused || h->fnodes)))
+    resident_plan = start_resident(h, *mesh);
   h->dp.tile_nodes = (params->kernel == FVDBM_KERNEL_TILE) ? 1 : 0;
   p.N = hp.N;
   p.Np = hp.Np;
@@ -689,6 +818,7 @@ static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, c
   }
   if ((rc = dalloc<float>(h, &h->stage, size_t(hp.q) * std::max(hp.N, hp.F))) != FVDBM_OK)
     return create_fail(h, rc);
+  if ((rc = make_resident(h, resident_plan)) != FVDBM_OK) return create_fail(h, rc);
   if ((rc = dalloc(h, &h->d_cell_new, hp.cell_new.size(), &hp.cell_new)) != FVDBM_OK)
     return create_fail(h, rc);
 
@@ -1059,6 +1189,11 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   h->in_ok = false;
   if (n_steps == 1 && h->hp.N > 0) CK(cudaEventRecord(h->in_ready, h->stream));
   int n = n_steps;
+  if (n >= (h->hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge) && !h->persist && resident_ready(h)) {
+    int rc = run_resident(h, n);
+    if (rc != FVDBM_OK) return rc;
+    n = 0;
+  }
   if (n >= kGraphSteps && h->hp.N > 0 && !h->persist) {
     int rc = ensure_nodes(h);  // outside the capture
     if (rc != FVDBM_OK) return rc;

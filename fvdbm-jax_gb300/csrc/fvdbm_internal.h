@@ -159,6 +159,70 @@ struct BatchSegs {
   const int32_t* node_ptr;
 };
 
+// Tables of the resident step (resident.cu, resident_plan.cpp): one part of
+// the cells per thread block, every index local to its block (own cells,
+// padded to a multiple of 32, then halo cells, then ghost entries).
+struct ResidentBlock {
+  int own_off, nown;      // own cells [own_off, own_off + nown) of dev / exp / hf / inv_area
+  int halo_off, nhalo;    // imported cells of halo_dev / halo_exp
+  int st_off, nst;        // distinct node-stencil cells (st_loc: local cell index)
+  int nd_off, nn;         // computed boundary nodes of nd / nd_sw
+  int fz_off, nf;         // frozen nodes (after the computed ones in the local node order)
+  int gh_off, ng;         // ghost entries of gh
+  int last_st;            // stencil index of the cell that padded node entries read
+  int en_off, ne;         // node entries of en_st / en_w
+  int pad;
+};
+
+struct ResidentPlan {
+  bool ok = false;
+  int n_export = 0;                    // exported cells of all blocks
+  int max_own = 0, stride = 0, max_nodes = 0, max_st = 0;
+  int max_table = 0;                   // words of a block's tables in shared memory
+  int cell_threads = 0, threads = 0;   // of a block (resident_threads)
+  std::vector<ResidentBlock> block;
+  std::vector<int32_t> dev, exp;       // device cell and export slot (-1: none) of each own cell
+  std::vector<int32_t> cls;            // per group of 32 own cells: 0 interior, 1 with halo faces or
+                                       // exports, 2 with ghosts
+  std::vector<uint32_t> hf;            // face slots (rows in resident.cu) with local neighbour indices
+  std::vector<float> inv_area;
+  std::vector<int32_t> halo_dev, halo_exp;
+  std::vector<int32_t> st_loc;
+  std::vector<int32_t> nd;             // {device node, type | padded << 2 | owner << 3, first entry, entries}
+  std::vector<float> nd_sw;
+  std::vector<uint32_t> en_st;         // stencil index | ND_NEQ_ZERO
+  std::vector<float> en_w;
+  std::vector<int32_t> fz_dev;
+  std::vector<int32_t> gh;             // {own cell, node a, node b, bits of the distance ratio}
+};
+void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
+                    ResidentPlan& rp);
+void resident_threads(int max_own, int* cell_threads, int* threads);
+
+// Device view of the same; ex holds two buffers of ResidentPlan::n_export
+// cells, each cell as 16-byte words of three pdfs and the step's tag.
+struct DevResident {
+  int n_blocks, threads, cell_threads, n_export, stride, max_nodes, max_st;
+  size_t smem;
+  const void* kern;
+  const ResidentBlock* block;
+  const int* dev;
+  const int* exp;
+  const int* cls;
+  const unsigned* hf;
+  const float* inv_area;
+  const int* halo_dev;
+  const int* halo_exp;
+  const int* st_loc;
+  const int4* nd;
+  const float* nd_sw;
+  const unsigned* en_st;
+  const float* en_w;
+  const int* fz_dev;
+  const int4* gh;
+  uint4* ex;
+};
+
 // Build the plan; returns an empty string on success, else the reason.
 std::string build_plan(const void* mesh, const void* params, HostPlan& hp,
                        const BatchSegs* segs = nullptr);
@@ -290,6 +354,15 @@ cudaError_t launch_fused_nodes(const DevPlan& p, const float* fin, float* fout, 
 // n_steps steps in one cooperative launch; f0 is the current buffer; bar is
 // one device int (zeroed by the launch)
 cudaError_t launch_persist(const DevPlan& p, float* f0, float* f1, int n_steps, int* bar, cudaStream_t s);
+// Resident step (resident.cu): n_steps steps in one cooperative launch from
+// fin; the last two states go to f_prev and f_last, the nodes of the last step
+// to p.node_*, and the stencil macros of f_last to p.cprod.  tag: the exchange
+// tags of the call's steps are tag + 1 .. tag + n_steps - 1 (never reused with
+// the same exchange buffer).  prepare_resident: threads and shared memory for the
+// plan, and whether the device can hold the grid.
+cudaError_t prepare_resident(const DevPlan& p, const ResidentPlan& rp, DevResident& r, bool* fits);
+cudaError_t launch_resident(const DevPlan& p, const DevResident& r, const float* fin, float* f_prev, float* f_last,
+                            int n_steps, unsigned tag, cudaStream_t s);
 // record the stencil macros of f (after an upload of the cell pdfs)
 cudaError_t launch_stencil_macros(const DevPlan& p, const float* f, cudaStream_t s);
 // the whole step in one launch (node blocks then cell blocks, see kernels.cu)

@@ -42,15 +42,15 @@ std::vector<int32_t> morton_order(const float* xy, int N) {
   }
   const double span = std::max(double(x1 - x0), double(y1 - y0));
   const double s = span > 0 ? 65535.0 / span : 0.0;
-  std::vector<std::pair<uint32_t, int32_t>> key(N);
+  std::vector<uint64_t> key(N);  // Z-order code, then the cell
   for (int i = 0; i < N; ++i) {
     uint32_t qx = uint32_t(std::min(65535.0, std::max(0.0, (xy[2 * i] - x0) * s)));
     uint32_t qy = uint32_t(std::min(65535.0, std::max(0.0, (xy[2 * i + 1] - y0) * s)));
-    key[i] = {spread16(qx) | (spread16(qy) << 1), i};
+    key[i] = (uint64_t(spread16(qx) | (spread16(qy) << 1)) << 32) | uint32_t(i);
   }
   std::sort(key.begin(), key.end());
   std::vector<int32_t> order(N);
-  for (int i = 0; i < N; ++i) order[i] = key[i].second;
+  for (int i = 0; i < N; ++i) order[i] = int32_t(key[i]);
   return order;
 }
 
@@ -448,19 +448,21 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
 
   // ---- faces in device order (by lowest slot cell)
   {
-    std::vector<std::pair<int64_t, int32_t>> fk(F);
+    // counting sort by the lowest slot cell (faces without one last), stable
+    std::vector<int32_t> start(size_t(N) + 2, 0), key(F);
     for (int f = 0; f < F; ++f) {
-      int64_t a = cnew(m.face_cells[2 * f]), b = cnew(m.face_cells[2 * f + 1]);
-      int64_t lo = (a < 0) ? b : (b < 0 ? a : std::min(a, b));
-      if (lo < 0) lo = int64_t(1) << 40;
-      fk[f] = {lo * (int64_t(F) + 1) + f, f};
+      const int32_t a = cnew(m.face_cells[2 * f]), b = cnew(m.face_cells[2 * f + 1]);
+      const int32_t lo = (a < 0) ? b : (b < 0 ? a : std::min(a, b));
+      key[f] = lo < 0 ? N : lo;
+      ++start[key[f] + 1];
     }
-    std::sort(fk.begin(), fk.end());
+    for (int i = 0; i <= N; ++i) start[i + 1] += start[i];
     hp.face_old.resize(F);
     hp.face_new.resize(F);
-    for (int j = 0; j < F; ++j) {
-      hp.face_old[j] = fk[j].second;
-      hp.face_new[fk[j].second] = j;
+    for (int f = 0; f < F; ++f) {
+      const int32_t j = start[key[f]]++;
+      hp.face_old[j] = f;
+      hp.face_new[f] = j;
     }
   }
   hp.fs0.resize(F);
@@ -594,7 +596,7 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
   // ---- tile tables: per tile the nodes its ghost faces need (plus owner-only
   // computed nodes that no ghost face uses), their stencil entries, and the
   // ghost end nodes as tile-local indices
-  if (hp.fusable && N > 0) {
+  if (hp.fusable && N > 0 && (pr.kernel == FVDBM_KERNEL_TILE || pr.kernel == FVDBM_KERNEL_TILE_SPLIT)) {
     const int NT = (N + TILE - 1) / TILE;
     const int G = int(hp.gh_a.size());
     std::vector<char> referenced(hp.M, 0);
@@ -672,7 +674,7 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
   // single-launch schedule: ticket -> work item (>= 0 cell block, < 0 node
   // block -(b+1)).  Node blocks are spread evenly over the first two thirds of
   // the ghost-free cell blocks; the cell blocks with ghost faces come last.
-  if (hp.fusable && N > 0) {
+  if (hp.fusable && N > 0 && pr.kernel == FVDBM_KERNEL_ONE) {
     std::vector<int32_t> free_blocks, ghost_blocks;
     for (int b = 0; b < int(hp.cblk_ghost.size()); ++b)
       (hp.cblk_ghost[b] ? ghost_blocks : free_blocks).push_back(b);

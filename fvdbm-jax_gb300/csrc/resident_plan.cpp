@@ -1,0 +1,300 @@
+// Host tables of the resident step (resident.cu): the cells are cut into
+// compact parts, one per thread block, and every index a block uses during a
+// run of steps becomes local to it: its own cells, then the halo cells it
+// imports from other blocks, then one ghost entry per ghost face.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "fvdbm_internal.h"
+
+namespace fvdbm {
+
+namespace {
+
+struct Point {
+  float x[2];
+  int32_t id;
+};
+
+// Recursive bisection of pts[a, b) (device cells) into parts [p0, p0 + parts)
+// of equal size, each cut across the longer side of its bounding box: compact
+// parts keep the halos short.  Without coordinates the device order is cut.
+void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, std::vector<int32_t>& part_end) {
+  if (parts == 1) {
+    part_end[p0] = b;
+    return;
+  }
+  const int left = parts / 2;
+  const int mid = a + int(int64_t(b - a) * left / parts);
+  if (xy) {
+    float lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
+    for (int i = a; i < b; ++i)
+      for (int d = 0; d < 2; ++d) {
+        lo[d] = std::min(lo[d], pts[i].x[d]);
+        hi[d] = std::max(hi[d], pts[i].x[d]);
+      }
+    const int d = hi[0] - lo[0] >= hi[1] - lo[1] ? 0 : 1;
+    std::nth_element(pts.begin() + a, pts.begin() + mid, pts.begin() + b, [d](const Point& u, const Point& v) {
+      return u.x[d] != v.x[d] ? u.x[d] < v.x[d] : u.id < v.id;
+    });
+  }
+  bisect(xy, pts, a, mid, p0, left, part_end);
+  bisect(xy, pts, mid, b, p0 + left, parts - left, part_end);
+}
+
+}  // namespace
+
+void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
+                    ResidentPlan& rp) {
+  rp = ResidentPlan{};
+  const int N = hp.N, H = hp.hrows;
+  if (N == 0 || !hp.fusable || hp.K != 3 || n_blocks < 1) return;
+  // the kernel drops terms that are +-0 for finite geometry
+  auto f32 = [](uint32_t u) {
+    float x;
+    std::memcpy(&x, &u, 4);
+    return x;
+  };
+  for (size_t g = 0; g < hp.hf.size() / (size_t(H) * 32); ++g)
+    for (size_t i = 3 * 32; i < size_t(H) * 32; ++i)
+      if (!std::isfinite(f32(hp.hf[g * H * 32 + i]))) return;
+  for (float a : hp.inv_area)
+    if (!std::isfinite(a)) return;
+  const bool lw = hp.scheme == FVDBM_LAX_WENDROFF, sc = hp.variant == FVDBM_VARIANT_FACE_SCALE;
+  const int NP = hp.q == 13 ? 6 : 4;
+  const int R = hp.fast ? H : 3 * ((lw ? 5 + NP : 4) + (sc ? 1 : 0));
+  const float* xy = m.cell_xy;
+  for (int64_t i = 0; xy && i < 2 * int64_t(N); ++i)
+    if (!std::isfinite(xy[i])) xy = nullptr;
+  auto hfi = [&](int i, int row) { return size_t(i >> 5) * size_t(H) * 32 + size_t(row) * 32 + (i & 31); };
+
+  // ---- parts
+  const int B = std::min(n_blocks, N);
+  std::vector<int32_t> ids(N), part_end(B), part(N), loc(N);
+  {
+    std::vector<Point> pts(N);
+    for (int i = 0; i < N; ++i) {
+      const int32_t c = hp.cell_old[i];
+      pts[i] = Point{{xy ? xy[2 * size_t(c)] : 0.0f, xy ? xy[2 * size_t(c) + 1] : 0.0f}, i};
+    }
+    bisect(xy != nullptr, pts, 0, N, 0, B, part_end);
+    for (int i = 0; i < N; ++i) ids[i] = pts[i].id;
+  }
+  for (int t = 0, i = 0; t < B; ++t)
+    for (; i < part_end[t]; ++i) part[ids[i]] = t;
+
+  // ---- what each block imports: the cells across its faces and the stencil
+  // cells of the boundary nodes its ghost faces read.  A node that no ghost
+  // face reads belongs to the block of its first stencil cell.
+  std::vector<std::vector<int32_t>> imp(B), nodes(B);
+  std::vector<std::vector<int32_t>> ghost_cells(B);
+  std::vector<int32_t> mark(N, -1), nmark(hp.M, -1);
+  std::vector<char> node_used(hp.M, 0);
+  for (int c = 0; c < N; ++c)
+    for (int k = 0; k < 3; ++k) {
+      const int32_t code = int32_t(hp.hf[hfi(c, k)]);
+      if (code & HF_GHOST) node_used[hp.gh_a[code >> HF_SHIFT]] = node_used[hp.gh_b[code >> HF_SHIFT]] = 1;
+    }
+  std::vector<std::vector<int32_t>> extra(B);
+  for (int d = 0; d < hp.Mc; ++d)
+    if (!node_used[d])
+      extra[hp.nd_ptr[d + 1] > hp.nd_ptr[d] ? part[hp.nd_cell[hp.nd_ptr[d]] & ~ND_NEQ_ZERO] : 0].push_back(d);
+  std::vector<char> links(size_t(B) * B, 0);  // links[t * B + u]: t imports from u
+  for (int t = 0; t < B; ++t) {
+    auto need = [&](int32_t c) {
+      if (part[c] != t && mark[c] != t) {
+        mark[c] = t;
+        imp[t].push_back(c);
+        links[size_t(t) * B + part[c]] = 1;
+      }
+    };
+    auto node = [&](int32_t d) {
+      if (nmark[d] == t) return;
+      nmark[d] = t;
+      nodes[t].push_back(d);
+      if (d >= hp.Mc) return;
+      for (int e = hp.nd_ptr[d]; e < hp.nd_ptr[d + 1]; ++e) need(int32_t(hp.nd_cell[e] & ~ND_NEQ_ZERO));
+      if (hp.nd_npad[d] > 0) need(hp.last_cell_new);
+    };
+    for (int i = t ? part_end[t - 1] : 0; i < part_end[t]; ++i)
+      for (int k = 0; k < 3; ++k) {
+        const int32_t code = int32_t(hp.hf[hfi(ids[i], k)]);
+        if (code & HF_GHOST) {
+          node(hp.gh_a[code >> HF_SHIFT]);
+          node(hp.gh_b[code >> HF_SHIFT]);
+        } else {
+          need(code >> HF_SHIFT);
+        }
+      }
+    for (int32_t d : extra[t]) node(d);
+  }
+  // a block may overwrite an exported value only once its reader has moved
+  // on, which it learns from the reader's own exports: every link goes both
+  // ways (a one-way link gets one cell to read back)
+  for (int t = 0; t < B; ++t)
+    for (int u = 0; u < B; ++u)
+      if (links[size_t(t) * B + u] && !links[size_t(u) * B + t]) {
+        const int32_t c = ids[t ? part_end[t - 1] : 0];
+        imp[u].push_back(c);
+        links[size_t(u) * B + t] = 1;
+      }
+
+  // ---- local order: one interior cell per cell thread (work that waits for
+  // nothing), then the cells with halo faces or exports, those with ghost faces, and
+  // the remaining interior cells; export slots in that order
+  std::vector<char> exported(N, 0);
+  for (int t = 0; t < B; ++t)
+    for (int32_t c : imp[t]) exported[c] = 1;
+  std::vector<int32_t> slot(N, -1);
+  // (an exported cell waits for the imports too: its next value overwrites
+  // the one that its readers must have taken)
+  std::vector<char> kind(exported);
+  for (int c = 0; c < N; ++c)
+    for (int k = 0; k < 3; ++k) {
+      const int32_t code = int32_t(hp.hf[hfi(c, k)]);
+      if (code & HF_GHOST)
+        kind[c] = 2;
+      else if (part[code >> HF_SHIFT] != part[c])
+        kind[c] = std::max<char>(kind[c], 1);
+    }
+  for (int t = 0; t < B; ++t) rp.max_own = std::max(rp.max_own, part_end[t] - (t ? part_end[t - 1] : 0));
+  resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
+  int off = 0;
+  for (int t = 0; t < B; ++t) {
+    const int a = t ? part_end[t - 1] : 0, b = part_end[t];
+    std::sort(ids.begin() + a, ids.begin() + b);
+    const auto first = ids.begin() + a, last = ids.begin() + b;
+    const auto in_end = std::stable_partition(first, last, [&](int32_t c) { return kind[c] == 0; });
+    std::stable_partition(in_end, last, [&](int32_t c) { return kind[c] == 1; });
+    const int inner = int(in_end - first);
+    if (inner > rp.cell_threads) std::rotate(ids.begin() + a + rp.cell_threads, ids.begin() + a + inner, ids.begin() + b);
+    ResidentBlock mb{};
+    mb.own_off = off;
+    mb.nown = b - a;
+    for (int i = a; i < b; ++i) {
+      loc[ids[i]] = i - a;
+      if (exported[ids[i]]) slot[ids[i]] = rp.n_export++;
+    }
+    off += (b - a + 31) / 32 * 32;
+    rp.block.push_back(mb);
+  }
+  rp.dev.assign(off, -1);
+  rp.exp.assign(off, -1);
+  rp.cls.assign(off / 32, 0);
+  rp.hf.assign(size_t(off / 32) * R * 32, 0u);
+  auto ri = [&](int i, int row) { return size_t(i >> 5) * size_t(R) * 32 + size_t(row) * 32 + (i & 31); };
+  auto bits = [](float x) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    return u;
+  };
+  const HfRows HR{3, hp.scheme, hp.variant};
+  if (hp.fv) rp.inv_area.assign(off, 0.0f);
+  std::vector<int32_t> hloc(N, -1), nloc(hp.M, -1), sloc(N, -1);
+  std::vector<char> node_owned(hp.M, 0);
+  bool finite_t = true;
+  for (int t = 0; t < B; ++t) {
+    ResidentBlock& mb = rp.block[t];
+    const int a = t ? part_end[t - 1] : 0, pad = (mb.nown + 31) / 32 * 32;
+    std::sort(imp[t].begin(), imp[t].end(), [&](int32_t x, int32_t y) { return slot[x] < slot[y]; });
+    mb.halo_off = int(rp.halo_dev.size());
+    mb.nhalo = int(imp[t].size());
+    for (int j = 0; j < mb.nhalo; ++j) {
+      rp.halo_dev.push_back(imp[t][j]);
+      rp.halo_exp.push_back(slot[imp[t][j]]);
+      hloc[imp[t][j]] = pad + j;
+    }
+    auto local = [&](int32_t c) { return part[c] == t ? loc[c] : hloc[c]; };
+    // boundary nodes: computed first, then frozen
+    std::stable_partition(nodes[t].begin(), nodes[t].end(), [&](int32_t d) { return d < hp.Mc; });
+    mb.nd_off = int(rp.nd.size() / 4);
+    mb.fz_off = int(rp.fz_dev.size());
+    mb.st_off = int(rp.st_loc.size());
+    mb.last_st = 0;
+    mb.en_off = int(rp.en_st.size());
+    std::vector<int32_t> touched;
+    auto st = [&](int32_t c) {
+      if (sloc[c] < 0) {
+        sloc[c] = mb.nst++;
+        rp.st_loc.push_back(local(c));
+        touched.push_back(c);
+      }
+      return sloc[c];
+    };
+    for (size_t j = 0; j < nodes[t].size(); ++j) {
+      const int32_t d = nodes[t][j];
+      nloc[d] = int(j);
+      if (d >= hp.Mc) {
+        rp.fz_dev.push_back(d);
+        ++mb.nf;
+        continue;
+      }
+      ++mb.nn;
+      if (hp.nd_npad[d] > 0) mb.last_st = st(hp.last_cell_new);
+      rp.nd.push_back(d);
+      rp.nd.push_back(hp.nd_type[d] | (hp.nd_npad[d] > 0 ? 4 : 0) | (node_owned[d] ? 0 : 8));
+      rp.nd.push_back(int(rp.en_st.size()));
+      rp.nd.push_back(hp.nd_ptr[d + 1] - hp.nd_ptr[d]);
+      rp.nd_sw.push_back(hp.nd_sumw[d]);
+      node_owned[d] = 1;
+      for (int e = hp.nd_ptr[d]; e < hp.nd_ptr[d + 1]; ++e) {
+        const uint32_t code = hp.nd_cell[e];
+        rp.en_st.push_back(uint32_t(st(int32_t(code & ~ND_NEQ_ZERO))) | (code & ND_NEQ_ZERO));
+        rp.en_w.push_back(hp.nd_w[e]);
+      }
+    }
+    for (int32_t c : touched) sloc[c] = -1;
+    mb.ne = int(rp.en_st.size()) - mb.en_off;
+    // face slots with local indices; ghost faces get their own entries
+    mb.gh_off = int(rp.gh.size() / 4);
+    for (int l = 0; l < mb.nown; ++l) {
+      const int32_t c = ids[a + l];
+      const int g = mb.own_off + l;
+      rp.dev[g] = c;
+      rp.exp[g] = slot[c];
+      if (hp.fv) rp.inv_area[g] = hp.inv_area[c];
+      rp.cls[g / 32] = std::max<int32_t>(rp.cls[g / 32], kind[c]);
+      for (int row = 3; row < (hp.fast ? H : 12); ++row) rp.hf[ri(g, row)] = hp.hf[hfi(c, row)];
+      if (!hp.fast)
+        for (int k = 0; k < 3; ++k) {
+          if (lw) {
+            // the interpolation weights' quotients (xi.n * dt) / D2, in the
+            // float32 operations of the per-step kernels
+            rp.hf[ri(g, 12 + k)] = hp.hf[hfi(c, HR.r(k))];
+            const float nx = f32(hp.hf[hfi(c, HR.nx(k))]), ny = f32(hp.hf[hfi(c, HR.ny(k))]);
+            const float D2 = f32(hp.hf[hfi(c, HR.d2(k))]);
+            const float v[6] = {nx, ny, nx + ny, ny - nx, 2.0f * nx, 2.0f * ny};
+            for (int j = 0; j < NP; ++j) {
+              const float t = (v[j] * pr.delta_t) / D2;
+              if (!std::isfinite(t)) finite_t = false;
+              rp.hf[ri(g, 15 + 3 * j + k)] = bits(t);
+            }
+          }
+          if (sc) rp.hf[ri(g, 3 * (lw ? 5 + NP : 4) + k)] = hp.hf[hfi(c, HR.sc(k))];
+        }
+      for (int k = 0; k < 3; ++k) {
+        const int32_t code = int32_t(hp.hf[hfi(c, k)]);
+        int32_t idx;
+        if (code & HF_GHOST) {
+          const int gi = code >> HF_SHIFT;
+          int32_t rbits;
+          std::memcpy(&rbits, &hp.gh_r[gi], 4);
+          idx = pad + mb.nhalo + mb.ng++;
+          const int32_t row4[4] = {l, nloc[hp.gh_a[gi]], nloc[hp.gh_b[gi]], rbits};
+          rp.gh.insert(rp.gh.end(), row4, row4 + 4);
+        } else {
+          idx = local(code >> HF_SHIFT);
+        }
+        rp.hf[ri(g, k)] = uint32_t((code & HF_SLOT1) | (idx << HF_SHIFT));
+      }
+    }
+    rp.stride = std::max(rp.stride, pad + mb.nhalo + mb.ng);
+    rp.max_nodes = std::max(rp.max_nodes, mb.nn + mb.nf);
+    rp.max_st = std::max(rp.max_st, mb.nst);
+    rp.max_table = std::max(rp.max_table, 8 * mb.nn + 4 * mb.ng + 2 * mb.ne + mb.nst + mb.nhalo);
+  }
+  rp.ok = finite_t;
+}
+
+}  // namespace fvdbm

@@ -63,7 +63,10 @@ extern "C" {
 #define FVDBM_KERNEL_AUTO 0       /* fastest family the mesh allows (FUSED_NODES from 2^18 cells,
                                      FUSED below and for D2Q13, STAGED when the fused kernels
                                      cannot run: not triangles, padded or foreign face slots,
-                                     per-q flux scale) */
+                                     per-q flux scale).  Runs of several steps (fvdbm_step with
+                                     n_steps >= 8) of a mesh whose state fits on the chip (about
+                                     400,000 D2Q9 triangles) take one launch, with the same
+                                     results; FAST does too */
 #define FVDBM_KERNEL_STAGED 1     /* node BC + face flux + cell gather (3 kernels) */
 #define FVDBM_KERNEL_FUSED 2      /* node BC + fused cell kernel (2 kernels; triangles) */
 #define FVDBM_KERNEL_TILE 3       /* persistent tile kernel, nodes evaluated in-tile (1 kernel) */
@@ -72,9 +75,9 @@ extern "C" {
 #define FVDBM_KERNEL_BATCH 6      /* (reported by fvdbm_get_info) packed batch: node BC + fused cell kernel */
 #define FVDBM_KERNEL_FUSED_NODES 7 /* fused cell kernel that also updates the boundary nodes of the
                                       next step (1 kernel) */
-#define FVDBM_KERNEL_PERSIST 8    /* all the steps of one fvdbm_step call in one cooperative launch:
-                                     nodes, grid barrier, cells, grid barrier per step (triangles;
-                                     for meshes whose launches are short) */
+#define FVDBM_KERNEL_PERSIST 8    /* all the steps of one fvdbm_step call in one cooperative launch
+                                     (triangles): with the state on the chip when it fits, else
+                                     nodes, grid barrier, cells, grid barrier per step */
 #define FVDBM_KERNEL_FAST 9       /* FUSED_NODES with contracted float32 arithmetic (multiply-adds,
                                      reciprocals of the lattice constants, no literal paths for
                                      non-finite values): bitwise reproducible run to run, within a

@@ -1,0 +1,96 @@
+"""Runs of several steps in one launch with the state on the chip against the
+same number of single staged steps, bit for bit: one to many blocks, one and
+several cells per thread, both lattices and flux schemes, the finite-volume
+update and the cos stencil, runs that follow one another and single steps in
+between, and states with non-finite values (whose steps take the literal form
+block by block)."""
+import numpy as np
+import pytest
+
+import goldens as G
+from test_gpu_random_state import KEYS, SPECIAL
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(cells, flux, lattice="D2Q9", mesh="cavity", special=0.0, cos=False, seed=3):
+    from fvdbm_jax_gb300 import D2Q9, D2Q13, Mesher, meshgen
+    if mesh == "cavity":
+        raw = meshgen.cavity(n=int(round((cells / 2) ** 0.5)) + 1, seed=seed)
+    else:
+        raw = meshgen.channel_cylinder(n_target=cells, seed=seed)
+    m = Mesher().import_meshpy(raw)
+    m.calc_mesh_properties()
+    dyn = (D2Q9 if lattice == "D2Q9" else D2Q13)(0.6, 0.25 * float(m.face_lengths.min()))
+    c, f, n = m.to_env(dyn, flux)
+    if cos:
+        f.stencil_variant = "cos"
+        f.alpha = np.random.default_rng(seed).uniform(0, 0.4, (f.n.shape[0], 1)).astype(np.float32)
+    for mk in (1, 2, 4, 5):
+        n = m.set_vel_node(n, mk, (0.0, 0.0))
+    n = m.set_vel_node(n, 3, (0.1, 0.0))
+    if mesh == "channel":
+        n = m.set_rho_node(n, 2, 1.0)
+    rng = np.random.default_rng(seed + 1)
+    pdf = np.asarray(c.pdf, np.float32)
+    pdf = (pdf * (1.0 + 0.1 * rng.standard_normal(pdf.shape))).astype(np.float32)
+    if special:
+        pick = rng.random(pdf.shape) < special
+        pdf[pick] = SPECIAL[rng.integers(0, SPECIAL.size, int(pick.sum()))]
+    c.pdf = pdf
+    return c, f, n
+
+
+def _same(a, b, what):
+    ga, gb = G.env_state(a), G.env_state(b)
+    for k in KEYS:
+        assert np.array_equal(ga[k], gb[k], equal_nan=True), (what, k)
+
+
+def _compare(cfn, runs, kernel, ref, fv=False):
+    from fvdbm_jax_gb300 import Environment
+    a, b = (Environment(*cfn, kernel=k, finite_volume=fv) for k in (kernel, ref))
+    a.init()
+    b.init()
+    for n in runs:
+        a.step(n)
+        for _ in range(n):
+            b.step()
+        _same(a, b, (kernel, n))
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("lattice", ["D2Q9", "D2Q13"])
+@pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
+@pytest.mark.parametrize("cells,mesh", [(2, "cavity"), (18, "cavity"), (98, "cavity"), (3200, "cavity"),
+                                        (60_000, "channel"), (96_000, "cavity")])
+def test_runs_match_single_steps(cells, mesh, flux, lattice):
+    _compare(_case(cells, flux, lattice, mesh), (4, 1, 7, 33), "auto", "staged")
+
+
+@pytest.mark.parametrize("kernel", ["auto", "persist"])
+@pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
+def test_cos_stencil_and_finite_volume(flux, kernel):
+    _compare(_case(5000, flux, cos=True), (5, 8), kernel, "staged")
+    _compare(_case(5000, flux), (5, 8), kernel, "staged", fv=True)
+
+
+def test_many_cells_per_thread():
+    """Beyond 2^18 cells (the single-launch family's node buffers) and near
+    the capacity of the blocks' shared memory."""
+    for cells in (270_000, 400_000):
+        _compare(_case(cells, "upwind"), (4, 1, 6), "auto", "fused")
+
+
+@pytest.mark.parametrize("lattice", ["D2Q9", "D2Q13"])
+@pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
+@pytest.mark.parametrize("share", [1e-4, 2e-3])
+def test_non_finite_states(share, flux, lattice):
+    _compare(_case(3200, flux, lattice, special=share), (6, 5), "auto", "staged")
+
+
+@pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
+@pytest.mark.parametrize("cells", [98, 3200, 120_000])
+def test_fast_family_runs_match_single_steps(cells, flux):
+    _compare(_case(cells, flux), (4, 1, 20), "fast", "fast")
