@@ -739,7 +739,9 @@ def _case_arrays(case, rho_in: float, rho_out: float):
     phib = np.zeros(F, np.float32)
     phib[open_] = (0.5 * ((nr[fno[open_, 0]] - rho_out) + (nr[fno[open_, 1]] - rho_out)) / d).astype(np.float32)
     wall = np.asarray(m.face_centers, np.float64)[bnd & ~open_]
-    return {"N": N, "F": F, "cf": cf, "cs": cs, "fc": fc, "fd": fd, "fL": fL, "fn": fnrm, "kind": kind,
+    cenT = np.ascontiguousarray(cen.T)
+    lo, hi = (cenT.min(1), cenT.max(1)) if N else (np.zeros(2), np.zeros(2))
+    return {"N": N, "F": F, "lo": lo, "hi": hi, "cf": cf, "cs": cs, "fc": fc, "fd": fd, "fL": fL, "fn": fnrm, "kind": kind,
             "phib": phib, "cen": cen, "area": area.astype(np.float32), "wall": wall.astype(np.float32),
             "rho_in": rho_in, "rho_out": rho_out, "has_open": bool(open_.any())}
 
@@ -863,8 +865,7 @@ def predict_cases(net, cases, rho_in, rho_out, batch_cells: int = 2_000_000, rto
             bins = torch.empty(ng, dtype=torch.int32, device=dev)
             count = torch.zeros(nb * len(grp), dtype=torch.int32, device=dev)
             for j, (k, go) in enumerate(zip(grp, gofs[:-1])):
-                cen = arr[k]["cen"]
-                lo, hi = cen.min(0), cen.max(0)
+                lo, hi = arr[k]["lo"], arr[k]["hi"]
                 sp = np.maximum(hi - lo, 1e-30)
                 chk(L.fvdbm_ws_bin_ids(arr[k]["N"], P(D[k]["cen"]), float(lo[0]), float(lo[1]), float(sp[0]),
                                        float(sp[1]), gg, P(bins[int(go):]), P(count[nb * j:]), st))

@@ -87,7 +87,9 @@ int fvdbm_mp_to_bf16(const float *x, uint16_t *y, size_t count, void *stream);
  * in float32, then in double over blocks, in a fixed order: bitwise
  * reproducible.  work: device scratch of at least
  * fvdbm_pcg_work_bytes(n) bytes.  *iters and *rel_res report the end state
- * (rel_res NaN: A was not positive definite or the input not finite). */
+ * (rel_res NaN: A was not positive definite or the input not finite).
+ * Systems of up to about 300,000 rows run in one cooperative launch;
+ * FVDBM_EDEVICE: a bounded wait in it gave up. */
 size_t fvdbm_pcg_work_bytes(int32_t n);
 int fvdbm_pcg(int32_t n, const int32_t *indptr, const int32_t *indices, const float *values, const float *b,
               float *x, int32_t max_iter, double rtol, int32_t check_every, void *work, size_t work_bytes,

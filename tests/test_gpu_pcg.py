@@ -86,3 +86,71 @@ def test_predict_cases_on_the_gpu_matches_the_host_path():
             assert g.shape == h.shape
             scale = np.abs(h).max(0)
             assert np.all(np.abs(g - h).max(0) <= 1e-3 * scale + 1e-6), (np.abs(g - h).max(0), scale)
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1025, 40_000, 155_648, 155_649, 311_296, 311_297])
+def test_pcg_sizes(n):
+    """One to many row groups per block and the launch-per-kernel form beyond
+    them: rows of 1 to 9 entries in any column order, entries out of range
+    (skipped), the residual it reports against float64, the same bits twice."""
+    import ctypes as C
+
+    import scipy.sparse as sp
+    import torch
+
+    from fvdbm_jax_gb300 import _native as nat
+    rng = np.random.default_rng(n)
+    m = 3 * n
+    i, j = rng.integers(0, n, m), rng.integers(0, n, m)
+    w = rng.uniform(0.1, 1.0, m)
+    A = sp.coo_matrix((-np.concatenate([w, w]), (np.concatenate([i, j]), np.concatenate([j, i]))), shape=(n, n)).tocsr()
+    A.setdiag(0.0)
+    A.eliminate_zeros()
+    A = (A + sp.diags(0.05 - np.asarray(A.sum(1)).reshape(-1))).tocsr().astype(np.float32)
+    A.sum_duplicates()
+    b = rng.standard_normal(n).astype(np.float32)
+    ix, v, ip = A.indices.astype(np.int32), A.data.copy(), A.indptr.astype(np.int32)
+    # an out-of-range entry at the end of the last row
+    ix, v = np.append(ix, np.int32(n + 5)), np.append(v, np.float32(1e9))
+    ip[-1] += 1
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (ip, ix, v, b)]
+    L = nat.lib()
+    wb = int(L.fvdbm_pcg_work_bytes(n))
+    outs = []
+    for _ in range(2):
+        work = torch.full((wb,), 7, dtype=torch.uint8, device="cuda")
+        x = torch.zeros(n, device="cuda")
+        it, rel = C.c_int32(0), C.c_double(0.0)
+        rc = L.fvdbm_pcg(n, *[t.data_ptr() for t in dev], x.data_ptr(), 2000, 1e-5, 7, work.data_ptr(), wb,
+                         torch.cuda.current_stream().cuda_stream, C.byref(it), C.byref(rel))
+        assert rc == 0
+        outs.append((x.cpu().numpy(), it.value, rel.value))
+    assert np.array_equal(outs[0][0], outs[1][0]) and outs[0][1:] == outs[1][1:]
+    xs, its, rel = outs[0]
+    assert its > 0 and its % 7 == 0 and rel <= 1e-5
+    true = np.linalg.norm(b - A.astype(np.float64) @ xs) / np.linalg.norm(b)
+    # the recurrence's residual drifts from the true one by rounding: a few
+    # hundred float32 ulps of |A||x| at most on these well-conditioned systems
+    assert true <= 1e-5 + 300 * 6e-8 * np.linalg.norm(abs(A).astype(np.float64) @ abs(xs)) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("bins", [1, 16, 300])
+def test_bin_rows(n, bins):
+    """Each bin's cells in ascending order, against a stable sort by bin."""
+    import torch
+
+    from fvdbm_jax_gb300 import _native as nat
+    rng = np.random.default_rng(n + bins)
+    b = rng.integers(0, bins, n).astype(np.int32)
+    start = np.concatenate([[0], np.cumsum(np.bincount(b, minlength=bins))]).astype(np.int32)
+    w = rng.uniform(size=bins).astype(np.float32)
+    dev = [torch.from_numpy(a).cuda() for a in (b, start, w)]
+    pcol, ucol = (torch.full((n,), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    pwt = torch.zeros(n, device="cuda")
+    nat.check(nat.lib().fvdbm_ws_bin_rows(n, bins, *[t.data_ptr() for t in dev], 7, 3, pcol.data_ptr(), pwt.data_ptr(),
+                                          ucol.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    order = np.argsort(b, kind="stable")
+    assert np.array_equal(pcol.cpu().numpy(), order + 7)
+    assert np.array_equal(pwt.cpu().numpy(), w[b[order]])
+    assert np.array_equal(ucol.cpu().numpy(), b + 3)
