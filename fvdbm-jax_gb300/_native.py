@@ -67,7 +67,8 @@ EXPORTS = ["fvdbm_create", "fvdbm_set_state", "fvdbm_step", "fvdbm_step_phase", 
            "fvdbm_mp_relu_bwd", "fvdbm_mp_spmm", "fvdbm_mp_mse_scratch", "fvdbm_mp_mse", "fvdbm_mp_adam",
            "fvdbm_mp_to_bf16", "fvdbm_mp_spmm_chunked", "fvdbm_pcg_work_bytes", "fvdbm_pcg",
            "fvdbm_ws_wall_distance", "fvdbm_ws_potential_rows", "fvdbm_ws_potential_grad", "fvdbm_ws_mesh_mean",
-           "fvdbm_ws_bin_ids", "fvdbm_ws_bin_rows"]
+           "fvdbm_ws_bin_ids", "fvdbm_ws_bin_rows", "fvdbm_mp_fused_scratch", "fvdbm_mp_layer_fwd",
+           "fvdbm_mp_layer_bwd", "fvdbm_mp_enc_fwd", "fvdbm_mp_enc_bwd", "fvdbm_mp_dec_fwd", "fvdbm_mp_dec_bwd"]
 
 
 def lib_path() -> str:
@@ -112,6 +113,14 @@ def lib(build_if_missing: bool = True) -> C.CDLL:
     L.fvdbm_mp_relu_bwd.argtypes = [u64, u64, u64, sz, u64]
     L.fvdbm_mp_spmm.argtypes = [u64, u64, u64, i32, u64, i32, u64, i32, u64]
     L.fvdbm_mp_spmm_chunked.argtypes = [u64, u64, i32, u64, u64, i32, u64, i32, u64, i32, u64, u64]
+    L.fvdbm_mp_fused_scratch.argtypes = [i32]
+    L.fvdbm_mp_fused_scratch.restype = sz
+    L.fvdbm_mp_layer_fwd.argtypes = [u64, i32] + [u64] * 9
+    L.fvdbm_mp_layer_bwd.argtypes = [u64, i32] + [u64] * 15 + [sz, u64]
+    L.fvdbm_mp_enc_fwd.argtypes = [u64, i32, i32, u64, u64, u64, u64, u64]
+    L.fvdbm_mp_enc_bwd.argtypes = [u64, i32] + [u64] * 6 + [i32, u64, u64, u64, sz, u64]
+    L.fvdbm_mp_dec_fwd.argtypes = [u64, i32, u64, u64, i32, u64, u64]
+    L.fvdbm_mp_dec_bwd.argtypes = [u64, u64, i32, u64, i32, u64, u64, u64, u64, sz, u64]
     L.fvdbm_mp_mse_scratch.argtypes = [sz]
     L.fvdbm_mp_mse_scratch.restype = sz
     L.fvdbm_mp_mse.argtypes = [u64, u64, u64, sz, C.c_float, u64, u64, sz, u64]

@@ -486,20 +486,38 @@ class MPNN:
         if with_targets:
             tn = (t - self.t_mu) / self.t_sd
             g["t"] = torch.from_numpy(np.ascontiguousarray(tn, np.float32)).to(d)
-        if work is not None and work["n"] >= n:
-            g["h"] = [a[:n] for a in work["h"]]
-            g["z"] = [a[:n] for a in work["z"]]
-            g["m"] = [a[:n] for a in work["m"]]
+        g["fused"] = self._fusable(g["agg"])
+        if work is not None and work["n"] >= n and work["fused"] == g["fused"]:
+            for k in ("h", "z", "m", "mask"):
+                g[k] = [a[:n] for a in work[k]]
             g["y"] = work["y"][:n]
-            for k in ("wscr", "dh", "dz", "dm", "dy", "mscr"):
+            for k in ("wscr", "dh", "dz", "dm", "dm2", "dy", "mscr"):
                 if work.get(k) is not None:
                     g[k] = work[k] if k in ("wscr", "mscr") else work[k][:n]
         else:
-            g["h"] = [torch.empty((n, H), device=d) for _ in range(self.layers + 1)]
-            g["z"] = [torch.empty((n, H), device=d) for _ in range(self.layers + 1)]
-            g["m"] = [torch.empty((n, H), device=d) for _ in range(self.layers)]
-            g["y"] = torch.empty((n, NOUT), device=d)
+            self._buffers(g)
         return g
+
+    def _fusable(self, agg) -> bool:
+        """The fused kernels (include/fvdbm_mpnn.h) take width 64 and gather
+        a layer's rows of its last forward and first backward stage inside:
+        both must be short (long ones go through the chunked aggregation)."""
+        return self.hidden == 64 and all(stages[-1]["pM"] is None and stages[0].get("pMt") is None for stages in agg)
+
+    def _buffers(self, g, train: bool = True):
+        """Activations of one pass over g's cells.  The fused kernels keep the
+        sign of the pre-activations (needed for training) and no messages."""
+        import torch
+        n, H, d = g["n"], self.hidden, self._dev
+        rows = lambda k: [torch.empty((n, H), device=d) for _ in range(k)]
+        g["h"] = rows(self.layers + 1)
+        g["y"] = torch.empty((n, NOUT), device=d)
+        g["z"], g["m"] = ([], []) if g["fused"] else (rows(self.layers + 1), rows(self.layers))
+        g["mask"] = []
+        if g["fused"]:
+            g["mask"] = [torch.empty((n, 2), dtype=torch.int32, device=d) for _ in range(self.layers + 1 if train else 1)]
+            if not train:
+                g["mask"] = g["mask"] * (self.layers + 1)
 
     def _spmm(self, M, rows, nch, partial, src, dst, accumulate):
         """dst (+)= M src over the CSR M: one thread per (row, feature), or in
@@ -514,6 +532,19 @@ class MPNN:
     def _forward(self, g):
         L, s, n, H = nat.lib(), self._stream(), g["n"], self.hidden
         P = self._p
+        if g["fused"]:
+            nat.check(L.fvdbm_mp_enc_fwd(P(g["x"]), n, NFEAT, self._w(0), self._b(0), P(g["h"][0]), P(g["mask"][0]), s))
+            for l in range(1, self.layers + 1):
+                src = g["h"][l - 1]
+                for st in g["agg"][l - 1][:-1]:
+                    self._spmm(st["M"], st["rows"], st["nchM"], st["pM"], src, st["tmp"], 0)
+                    src = st["tmp"]
+                M = g["agg"][l - 1][-1]["M"]
+                nat.check(L.fvdbm_mp_layer_fwd(P(g["h"][l - 1]), n, P(M[0]), P(M[1]), P(M[2]), P(src), self._w(l),
+                                               self._b(l), P(g["h"][l]), P(g["mask"][l]), s))
+            lo = self.layers + 1
+            nat.check(L.fvdbm_mp_dec_fwd(P(g["h"][-1]), n, self._w(lo), self._b(lo), NOUT, P(g["y"]), s))
+            return
         nat.check(L.fvdbm_mp_dense_fwd(P(g["x"]), NFEAT, 0, 0, n, self._w(0), self._b(0), H, 1, 0,
                                        P(g["z"][0]), P(g["h"][0]), s))
         for l in range(1, self.layers + 1):
@@ -535,14 +566,14 @@ class MPNN:
         and the loss scratch), sized for its cells."""
         import torch
         L, n, H = nat.lib(), g["n"], self.hidden
-        scratch_n = max(L.fvdbm_mp_wgrad_scratch(n, H, 2 * H), L.fvdbm_mp_wgrad_scratch(n, NOUT, H),
-                        L.fvdbm_mp_wgrad_scratch(n, H, NFEAT))
+        scratch_n = L.fvdbm_mp_fused_scratch(n) if g["fused"] else max(
+            L.fvdbm_mp_wgrad_scratch(n, H, 2 * H), L.fvdbm_mp_wgrad_scratch(n, NOUT, H),
+            L.fvdbm_mp_wgrad_scratch(n, H, NFEAT))
         if g.get("wscr") is None or g["wscr"].numel() * 4 < scratch_n:
             g["wscr"] = torch.empty((scratch_n + 3) // 4, dtype=torch.float32, device=self._dev)
         if g.get("dh") is None or g["dh"].shape[0] < n:
-            g["dh"] = torch.empty((n, H), device=self._dev)
-            g["dz"] = torch.empty((n, H), device=self._dev)
-            g["dm"] = torch.empty((n, H), device=self._dev)
+            for k in ("dh", "dm", "dm2" if g["fused"] else "dz"):
+                g[k] = torch.empty((n, H), device=self._dev)
         if g.get("dy") is None or g["dy"].shape[0] < n:
             g["dy"] = torch.empty((n, NOUT), device=self._dev)
             nb = L.fvdbm_mp_mse_scratch(n * NOUT)
@@ -555,6 +586,24 @@ class MPNN:
         ws, wsn = P(g["wscr"]), g["wscr"].numel() * 4
         lo = self.layers + 1
         G = self.G
+        if g["fused"]:
+            gw = lambda l: (self._w(l, G), self._b(l, G), ws, wsn, s)
+            dh = P(g["dh"])
+            nat.check(L.fvdbm_mp_dec_bwd(P(dy), P(g["h"][-1]), n, self._w(lo), NOUT, dh, *gw(lo)))
+            pend = (0, 0, 0, 0)  # rows still to be added to dh: the CSR of A^T's last stage, and its source
+            for l in range(self.layers, 0, -1):
+                stages, hp = g["agg"][l - 1], g["h"][l - 1]
+                M, src = stages[-1]["M"], (stages[-2]["tmp"] if len(stages) > 1 else hp)
+                grad = g["dm"] if l % 2 else g["dm2"]
+                nat.check(L.fvdbm_mp_layer_bwd(dh, n, *pend, P(g["mask"][l]), P(hp), P(M[0]), P(M[1]), P(M[2]), P(src),
+                                               self._w(l), P(grad), *gw(l)))
+                for st in reversed(stages[1:]):
+                    self._spmm(st["Mt"], st["cols"], st["nchMt"], st["pMt"], grad, st["gtmp"], 0)
+                    grad = st["gtmp"]
+                Mt = stages[0]["Mt"]
+                pend = (P(Mt[0]), P(Mt[1]), P(Mt[2]), P(grad))
+            nat.check(L.fvdbm_mp_enc_bwd(dh, n, *pend, P(g["mask"][0]), P(g["x"]), NFEAT, *gw(0)))
+            return
         nat.check(L.fvdbm_mp_dense_bwd_weight(P(dy), n, NOUT, P(g["h"][-1]), H, 0, 0, self._w(lo, G), self._b(lo, G),
                                               ws, wsn, s))
         nat.check(L.fvdbm_mp_dense_bwd_data(P(dy), n, NOUT, self._w(lo), H, 0, P(g["dh"]), 0, 0, s))
@@ -837,10 +886,8 @@ def predict_cases(net, cases, rho_in, rho_out, batch_cells: int = 2_000_000, rto
         groups.append(cur)
     nmax = max(sum(arr[k]["N"] for k in g) for g in groups)
     H = net.hidden
-    buf = {"h": [torch.empty((nmax, H), device=dev) for _ in range(net.layers + 1)],
-           "z": [torch.empty((nmax, H), device=dev) for _ in range(net.layers + 1)],
-           "m": [torch.empty((nmax, H), device=dev) for _ in range(net.layers)],
-           "y": torch.empty((nmax, NOUT), device=dev)}
+    buf = {"n": nmax, "fused": H == 64}  # (the cells' rows of every stage are short)
+    net._buffers(buf, train=False)
     preds = [None] * len(arr)
     for grp in groups:
         gofs = np.concatenate([[0], np.cumsum([arr[k]["N"] for k in grp])]).astype(np.int64)
@@ -893,8 +940,8 @@ def predict_cases(net, cases, rho_in, rho_out, batch_cells: int = 2_000_000, rto
                          "tmp": torch.empty((rows_b, H), device=dev)},
                         {"rows": ng, "cols": rows_b, "M": (ipu, ucol, ones, ipu, ipu), "nchM": ng, "pM": None,
                          "tmp": None}])
-        g = {"n": ng, "x": xn[o0:o0 + ng], "agg": agg, "h": [a_[:ng] for a_ in buf["h"]],
-             "z": [a_[:ng] for a_ in buf["z"]], "m": [a_[:ng] for a_ in buf["m"]], "y": buf["y"][:ng]}
+        g = {"n": ng, "x": xn[o0:o0 + ng], "agg": agg, "fused": buf["fused"], "y": buf["y"][:ng]}
+        g.update({k: [a_[:ng] for a_ in buf[k]] for k in ("h", "z", "m", "mask")})
         net._forward(g)
         y = g["y"].detach().cpu().numpy() * net.t_sd + net.t_mu
         for k, a0, a1 in zip(grp, gofs[:-1], gofs[1:]):

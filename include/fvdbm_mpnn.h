@@ -62,6 +62,38 @@ int fvdbm_mp_spmm_chunked(const int32_t *chunk_start, const int32_t *chunk_ptr, 
                           const int32_t *col, const float *wt, int32_t n, const float *h, int32_t d, float *out,
                           int32_t accumulate, float *partial, void *stream);
 
+/* Fused passes of the network at hidden width 64 (what MPNN runs at that
+ * width): the same quantities as the calls above, with the aggregation of the
+ * layer's last sparse stage inside.  Float arrays of width 64, bias and scratch
+ * are 16-byte aligned; mask holds the sign of the pre-activations, one bit per
+ * value ([n][2] words).
+ *   layer_fwd: m = sum_e wt[e] src[col[e]] over each row; z = [h | m] W^T + bias
+ *              (W [64][128]); hout = h + relu(z).
+ *   layer_bwd: dh += the pending rows sum_e pend_wt[e] pend_src[pend_col[e]]
+ *              (pend_src may be NULL); dz = dh where the mask is set;
+ *              dw = dz^T [h | m], dbias = column sums of dz; [dx | dm] = dz W;
+ *              dh += dx (in place).  dm must not be pend_src.
+ *   enc_fwd / enc_bwd: h = relu(x W^T + bias), din <= 16, and its dw, dbias.
+ *   dec_fwd / dec_bwd: y = h W^T + bias, dout <= 4; dh = dy W, dw, dbias.
+ * scratch: at least fvdbm_mp_fused_scratch(n) bytes. */
+size_t fvdbm_mp_fused_scratch(int32_t n);
+int fvdbm_mp_layer_fwd(const float *h, int32_t n, const int32_t *row_ptr, const int32_t *col, const float *wt,
+                       const float *src, const uint16_t *w, const float *bias, float *hout, uint32_t *mask,
+                       void *stream);
+int fvdbm_mp_layer_bwd(float *dh, int32_t n, const int32_t *pend_ptr, const int32_t *pend_col, const float *pend_wt,
+                       const float *pend_src, const uint32_t *mask, const float *h, const int32_t *row_ptr,
+                       const int32_t *col, const float *wt, const float *src, const uint16_t *w, float *dm, float *dw,
+                       float *dbias, float *scratch, size_t scratch_bytes, void *stream);
+int fvdbm_mp_enc_fwd(const float *x, int32_t n, int32_t din, const uint16_t *w, const float *bias, float *h,
+                     uint32_t *mask, void *stream);
+int fvdbm_mp_enc_bwd(const float *dh, int32_t n, const int32_t *pend_ptr, const int32_t *pend_col,
+                     const float *pend_wt, const float *pend_src, const uint32_t *mask, const float *x, int32_t din,
+                     float *dw, float *dbias, float *scratch, size_t scratch_bytes, void *stream);
+int fvdbm_mp_dec_fwd(const float *h, int32_t n, const uint16_t *w, const float *bias, int32_t dout, float *y,
+                     void *stream);
+int fvdbm_mp_dec_bwd(const float *dy, const float *h, int32_t n, const uint16_t *w, int32_t dout, float *dh, float *dw,
+                     float *dbias, float *scratch, size_t scratch_bytes, void *stream);
+
 /* Masked mean squared error: loss = sum mask (y - t)^2 / mask_total into
  * scratch[0] (double, device); dy = 2 mask (y - t) / mask_total.  mask may be
  * NULL (all ones).  scratch: at least fvdbm_mp_mse_scratch(count) bytes. */

@@ -117,3 +117,71 @@ def test_warm_start_needs_fewer_steps_than_uniform():
     sw, stw, restarted = WS.run_cases(warm, thr, every, cap, init=(np.concatenate(rho), np.concatenate(vel)))
     assert np.all(stp == 1) and np.all(stw == 1), (stp, stw)
     assert sw.sum() < sp_.sum(), (sw, sp_)
+
+
+@pytest.mark.parametrize("n", [8, 63, 64, 65, 127, 128, 129, 1000, 20_000])
+def test_fused_passes_match_separate_kernels(n, monkeypatch):
+    """The fused layers against the separate kernels at tile edges: the same
+    output and loss, bit for bit; gradients within 1e-4 of their scale (float32
+    sums in another order against the separate kernels' 21-bit operands)."""
+    from fvdbm_jax_gb300.warmstart import MPNN
+    smp, _ = _random_sample_sparse(n)
+    res = []
+    for fused in (True, False):
+        net = MPNN(seed=3, scales=("mesh", "mesh", "c5", 2))
+        if not fused:
+            monkeypatch.setattr(net, "_fusable", lambda agg: False)
+        g = net._upload([smp], True)
+        assert g["fused"] == fused
+        loss = float(net.loss_and_grads(g).item())
+        res.append((loss, g["y"].cpu().numpy(), net.grads()))
+    assert res[0][0] == res[1][0] and np.array_equal(res[0][1], res[1][1])
+    for (aw, ab), (bw, bb) in zip(res[0][2], res[1][2]):
+        assert np.abs(aw - bw).max() <= 1e-4 * max(np.abs(bw).max(), 1e-6)
+        assert np.abs(ab - bb).max() <= 1e-4 * max(np.abs(bb).max(), 1e-6)
+
+
+def _random_sample_sparse(n):
+    """As _random_sample, without the dense matrices (any n)."""
+    import scipy.sparse as sp
+
+    from fvdbm_jax_gb300.warmstart import NFEAT, Sample, _stage, grid_mean
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    j = rng.integers(0, n, n)
+    M = sp.csr_matrix((np.ones(4 * n), (np.concatenate([i, (i + 1) % n, i, j]), np.concatenate([(i + 1) % n, i, j, i]))),
+                      shape=(n, n))
+    M.data[:] = 1.0
+    A = (sp.diags(1.0 / np.asarray(M.sum(1)).reshape(-1)) @ M).tocsr().astype(np.float32)
+    xy = rng.uniform(0, 1, (n, 2))
+    aggs = [[_stage(A)], [_stage(A)]] + [[_stage(m) for m in grid_mean(xy, k, c)] for k, c in ((5, True), (2, False))]
+    return Sample(rng.standard_normal((n, NFEAT)).astype(np.float32), aggs,
+                  rng.standard_normal((n, 3)).astype(np.float32)), aggs
+
+
+@pytest.mark.parametrize("rows,chunks,d", [(1, 7, 64), (1, 8, 64), (3, 129, 64), (5, 1000, 64), (2, 300, 128), (4, 40, 7)])
+def test_long_rows_fold_in_order(rows, chunks, d):
+    """Chunked aggregation of long rows against the same float32 fold in numpy."""
+    import torch
+
+    from fvdbm_jax_gb300 import _native as nat
+    rng = np.random.default_rng(rows + chunks)
+    per = chunks * 64 - 13
+    n = 500
+    col = rng.integers(0, n, rows * per).astype(np.int32)
+    wt = rng.uniform(0, 1, rows * per).astype(np.float32)
+    h = rng.standard_normal((n, d)).astype(np.float32)
+    cs = np.concatenate([r * per + np.arange(0, per, 64) for r in range(rows)] + [[rows * per]]).astype(np.int32)
+    cp = (np.arange(rows + 1) * chunks).astype(np.int32)
+    t = [torch.from_numpy(a).cuda() for a in (cs, cp, col, wt, h)]
+    out = torch.zeros((rows, d), device="cuda")
+    part = torch.zeros((rows * chunks, d), device="cuda")
+    nat.check(nat.lib().fvdbm_mp_spmm_chunked(t[0].data_ptr(), t[1].data_ptr(), rows * chunks, t[2].data_ptr(),
+                                              t[3].data_ptr(), rows, t[4].data_ptr(), d, out.data_ptr(), 0,
+                                              part.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    p = part.cpu().numpy()
+    ref = np.zeros((rows, d), np.float32)
+    for r in range(rows):
+        for c in range(chunks):
+            ref[r] = ref[r] + p[r * chunks + c]
+    assert np.array_equal(out.cpu().numpy(), ref)
