@@ -98,6 +98,7 @@ struct Handle {
   cudaStream_t side = nullptr;  // highest priority: its blocks take SM slots as the step's retire
   cudaEvent_t in_ready = nullptr;
   bool in_ok = false;
+  bool stepping = false;  // the last call was fvdbm_step
   int* status_host = nullptr;  // page-locked copy of *status, filled on the stream before a sync
   int* d_rows = nullptr;       // [N] cell indices of a halo pack/unpack
   std::string err;
@@ -242,9 +243,11 @@ int upload_nodes(Handle* h) {
   return FVDBM_OK;
 }
 
-// Back-to-back steps use programmatic dependent launch between the node and
-// cell kernels (each waits for its predecessor before reading its output);
-// the first launch of a call follows whatever preceded it in the stream.
+// Steps use programmatic dependent launch between the node and cell kernels
+// (each waits for its predecessor before it reads what one wrote; anything else
+// before a call's first launch, a copy or a kernel that does not trigger its
+// dependents, is waited for in full).  Single steps one call at a time, 3.2k cells: 8.0
+// us, 9.8 without it on the first launch.
 // The plan with the node pointers of buffer a (read) and b (written).
 DevPlan with_nodes(const Handle* h, int a, int b) {
   DevPlan q = h->dp;
@@ -329,9 +332,8 @@ int enqueue_steps(Handle* h, int n) {
       h->node_last = h->node_cur;
       h->node_cur ^= 1;
     } else if (h->batch) {
-      CK(launch_nodes(h->dp, fin, h->stream, /*pdl=*/s > 0));
-      CK(launch_fused_batch(h->dp, fin, fout, h->stream, /*pdl=*/h->dp.NB > 0 || s > 0, h->batch_block,
-                            h->batch_waves));
+      CK(launch_nodes(h->dp, fin, h->stream, /*pdl=*/true));
+      CK(launch_fused_batch(h->dp, fin, fout, h->stream, /*pdl=*/true, h->batch_block, h->batch_waves));
     } else if (h->one) {
       CK(launch_step(h->dp, fin, fout, h->stream, /*pdl=*/s > 0));
     } else if (h->tile) {
@@ -339,11 +341,11 @@ int enqueue_steps(Handle* h, int n) {
       CK(launch_tile(h->dp, fin, fout, h->stream));
     } else {
       if (h->fused)
-        CK(launch_nodes_cp(h->dp, fin, h->stream, /*pdl=*/s > 0));
+        CK(launch_nodes_cp(h->dp, fin, h->stream, /*pdl=*/true));
       else
         CK(launch_nodes(h->dp, fin, h->stream, /*pdl=*/s > 0));
       if (h->fused) {
-        CK(launch_fused(h->dp, fin, fout, h->stream, /*pdl=*/h->dp.NB > 0 || s > 0));
+        CK(launch_fused(h->dp, fin, fout, h->stream, /*pdl=*/true));
       } else {
         CK(launch_face_flux(h->dp, fin, h->flux, h->stream));
         CK(launch_gather(h->dp, fin, h->flux, fout, h->stream));
@@ -403,7 +405,7 @@ int get_graph(Handle* h, int parity, cudaGraphExec_t* out) {
 
 // Tables of the resident step, when the state of this mesh fits on the chip:
 // planned beside the rest of fvdbm_create (start), then uploaded (make).
-std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh) {
+std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh, const float* case_dt) {
   int sms = 0, lim = 0;
   const HostPlan& hp = h->hp;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess ||
@@ -411,9 +413,9 @@ std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh) {
       int64_t(hp.N) * 2 * hp.q * 4 > int64_t(sms) * lim)
     return {};
   const int blocks = std::min(sms, (hp.N + kResidentCells - 1) / kResidentCells);
-  auto plan = [h, &mesh, blocks] {
+  auto plan = [h, &mesh, blocks, case_dt] {
     ResidentPlan rp;
-    build_resident(mesh, h->params, h->hp, blocks, rp);
+    build_resident(mesh, h->params, h->hp, blocks, case_dt, rp);
     return rp;
   };
   try {
@@ -645,8 +647,8 @@ static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, c
     h->batch = true;
     h->fused = h->tile = h->one = false;
   }
-  if (h->persist || params->kernel == FVDBM_KERNEL_FAST || (auto_family && (h->fused || h->fnodes)))
-    resident_plan = start_resident(h, *mesh);
+  if (h->persist || h->batch || params->kernel == FVDBM_KERNEL_FAST || (auto_family && (h->fused || h->fnodes)))
+    resident_plan = start_resident(h, *mesh, case_dt);
   h->dp.tile_nodes = (params->kernel == FVDBM_KERNEL_TILE) ? 1 : 0;
   p.N = hp.N;
   p.Np = hp.Np;
@@ -839,13 +841,10 @@ static int create_impl(const fvdbm_mesh_t* mesh, const fvdbm_params_t* params, c
   h->node_rho.assign(hp.P, 0.0f);
   h->node_vel.assign(size_t(2) * hp.P, 0.0f);
   if ((rc = upload_nodes(h)) != FVDBM_OK) return create_fail(h, rc);
-  {
-    std::vector<float> cells(size_t(Qh) * hp.N);
-    for (int c = 0; c < hp.N; ++c)
-      for (int q = 0; q < Qh; ++q) cells[size_t(c) * Qh + q] = W[q];
-    if ((rc = fvdbm_set_state(h, cells.data(), nullptr, nullptr, nullptr)) != FVDBM_OK)
-      return create_fail(h, rc);
-  }
+  RestPdf rest{};
+  std::memcpy(rest.v, W, size_t(Qh) * sizeof(float));
+  CR(launch_fill_rest(h->f[h->cur], rest, Qh, hp.N, h->stream));
+  if (h->fused && hp.q == 9) CR(launch_stencil_macros(h->dp, h->f[h->cur], h->stream));
   CR(cudaStreamSynchronize(h->stream));
   *handle = h;
   return FVDBM_OK;
@@ -1077,7 +1076,7 @@ int fvdbm_set_state(void* handle, const float* cell_pdf, const float* node_pdf, 
                     const float* node_vel) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   bool read_later = false;  // a page-locked source is read by the stream after this returns
@@ -1161,7 +1160,7 @@ int fvdbm_unpack_cells(void* handle, const int32_t* cells, int32_t n, const floa
 int fvdbm_set_cells_eq(void* handle, const float* rho, const float* vel) {
   if (!handle || !rho || !vel) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   if (h->hp.q != 9) return fail(h, FVDBM_EINVAL, "fvdbm_set_cells_eq supports D2Q9");
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
@@ -1187,7 +1186,11 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   if (n_steps < 0) return fail(h, FVDBM_EINVAL, "n_steps < 0");
   CK(cudaSetDevice(h->device));
   h->in_ok = false;
-  if (n_steps == 1 && h->hp.N > 0) CK(cudaEventRecord(h->in_ready, h->stream));
+  // (an event between two steps would part them: only a step that does not
+  // follow another one is marked for the read-back beside it)
+  const bool mark = n_steps == 1 && h->hp.N > 0 && !h->stepping;
+  if (mark) CK(cudaEventRecord(h->in_ready, h->stream));
+  h->stepping = true;
   int n = n_steps;
   if (n >= (h->hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge) && !h->persist && resident_ready(h)) {
     int rc = run_resident(h, n);
@@ -1208,7 +1211,7 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   }
   int rc = enqueue_steps(h, n);
   if (rc != FVDBM_OK) return rc;
-  h->in_ok = n_steps == 1 && h->hp.N > 0;
+  h->in_ok = mark;
   h->steps_done += n_steps;
   for (size_t s = 0; s < h->active.size(); ++s)
     if (h->active[s]) h->case_steps[s] += n_steps;
@@ -1343,6 +1346,7 @@ int fvdbm_sync(void* handle) {
 int fvdbm_get_cells(void* handle, float* pdf, float* rho, float* vel, float* pdf_eq) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
+  h->stepping = false;
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   const int N = hp.N;

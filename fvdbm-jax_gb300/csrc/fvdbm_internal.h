@@ -171,7 +171,7 @@ struct ResidentBlock {
   int gh_off, ng;         // ghost entries of gh
   int last_st;            // stencil index of the cell that padded node entries read
   int en_off, ne;         // node entries of en_st / en_w
-  int pad;
+  int cs;                 // the block's case (packed batch)
 };
 
 struct ResidentPlan {
@@ -196,7 +196,7 @@ struct ResidentPlan {
   std::vector<int32_t> gh;             // {own cell, node a, node b, bits of the distance ratio}
 };
 void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
-                    ResidentPlan& rp);
+                    const float* case_dt, ResidentPlan& rp);
 void resident_threads(int max_own, int* cell_threads, int* threads);
 
 // Device view of the same; ex holds two buffers of ResidentPlan::n_export
@@ -408,6 +408,10 @@ cudaError_t launch_gather_cells(const float* src, float* dst_aos, const int* cel
                                 cudaStream_t s, int q = Q);
 // the bounded-wait self-test (fvdbm_wait_selftest)
 cudaError_t launch_wait_selftest(const int* flag, int iters, int* status, cudaStream_t s);
+struct RestPdf {
+  float v[13];
+};
+cudaError_t launch_fill_rest(float* f, const RestPdf& w, int q, int N, cudaStream_t s);
 cudaError_t launch_pack_rows(const float* f, const int* cell_new, const int* idx, int n, float* buf,
                              cudaStream_t s, int q);
 cudaError_t launch_unpack_rows(float* f, const int* cell_new, const int* idx, int n, const float* buf,

@@ -946,6 +946,16 @@ __global__ void k_unpack_rows(float* __restrict__ f, const int* __restrict__ cel
   f[cell_base(cell_new[idx[k]], QQ) + size_t(q) * 32] = buf[t];
 }
 
+// The rest state: every cell's pdf = w (AoSoA).
+__global__ void __launch_bounds__(256) k_fill_rest(float* __restrict__ f, RestPdf w, int q, int N) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  float* o = f + cell_base(i, q);
+#pragma unroll
+  for (int k = 0; k < 13; ++k)
+    if (k < q) o[k * 32] = w.v[k];
+}
+
 // SoA [rows][Np] device order -> [N][rows] reference order.
 __global__ void k_soa_to_aos(const float* __restrict__ src, float* __restrict__ dst,
                              const int* __restrict__ cell_new, int N, int Np, int rows) {
@@ -1213,6 +1223,12 @@ cudaError_t launch_scatter_cells(const float* src_aos, float* dst, const int* ce
     k_aos_to_cells<13><<<blocks(N, 256), 256, 0, s>>>(src_aos, dst, cell_new, N);
   else
     k_aos_to_cells<Q><<<blocks(N, 256), 256, 0, s>>>(src_aos, dst, cell_new, N);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fill_rest(float* f, const RestPdf& w, int q, int N, cudaStream_t s) {
+  if (N == 0) return cudaSuccess;
+  k_fill_rest<<<blocks(N, 256), 256, 0, s>>>(f, w, q, N);
   return cudaGetLastError();
 }
 

@@ -507,8 +507,6 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
   }
 
   // ---- per-cell face slots: staged gather and fused half faces
-  hp.cf_face.assign(size_t(K) * hp.Np, 0);
-  hp.cf_sign.assign(size_t(K) * hp.Np, 0.0f);
   hp.fusable = (pr.variant != 2);
   for (int c = 0; c < N && hp.fusable; ++c)
     for (int k = 0; k < K; ++k) {
@@ -519,6 +517,12 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
         break;
       }
     }
+  // (only the staged gather reads the face lists)
+  const bool gather = !(hp.fusable && K == 3) || pr.kernel == FVDBM_KERNEL_STAGED;
+  if (gather) {
+    hp.cf_face.assign(size_t(K) * hp.Np, 0);
+    hp.cf_sign.assign(size_t(K) * hp.Np, 0.0f);
+  }
   const HfRows HR{K, pr.flux_scheme, pr.variant};
   const HfFastRows HX{K, pr.flux_scheme};
   hp.fast = pr.kernel == FVDBM_KERNEL_FAST && !segs;
@@ -542,8 +546,10 @@ std::string build_plan(const void* mesh_v, const void* params_v, HostPlan& hp, c
       const int32_t sg = m.cell_face_signs[int64_t(c) * K + k];
       const size_t s = size_t(k) * hp.Np + i;
       const int j = hp.face_new[f];
-      hp.cf_face[s] = j;
-      hp.cf_sign[s] = float(sg);
+      if (gather) {
+        hp.cf_face[s] = j;
+        hp.cf_sign[s] = float(sg);
+      }
       if (!hp.fusable) continue;
       const int32_t s0 = m.face_cells[2 * f], s1 = m.face_cells[2 * f + 1];
       const bool slot1 = (s1 == c);

@@ -131,7 +131,7 @@ __device__ __forceinline__ void load_rows(const unsigned* __restrict__ hf, int g
 // all finite.
 template <int LAT, int SCHEME, int VARIANT, bool FV, bool LIT>
 __device__ __forceinline__ void cell_step(const DevPlan& p, const float* f0, const unsigned* w, float ia,
-                                          const float* f, float* fn) {
+                                          float inv_tau, float dt, const float* f, float* fn) {
   using L = Lat<LAT>;
   constexpr int NQ = L::NQ, NP = L::NP;
   const float2 one2 = make_float2(p.one, p.one), m12 = make_float2(p.neg_one, p.neg_one);
@@ -192,7 +192,7 @@ __device__ __forceinline__ void cell_step(const DevPlan& p, const float* f0, con
 #pragma unroll
     for (int j = 0; j < NP; ++j) acc[j] = mul2(acc[j], make_float2(ia, ia));
   }
-  const float2 it2 = make_float2(p.inv_tau, p.inv_tau), dt2 = make_float2(p.dt, p.dt);
+  const float2 it2 = make_float2(inv_tau, inv_tau), dt2 = make_float2(dt, dt);
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     const int qp = pair_q(j), qm = qp + 2;
@@ -203,20 +203,21 @@ __device__ __forceinline__ void cell_step(const DevPlan& p, const float* f0, con
     fn[qp] = r.x;
     fn[qm] = r.y;
   }
-  fn[0] = f[0] + p.dt * (p.inv_tau * (eq[0] - f[0]) - acc0);
+  fn[0] = f[0] + dt * (inv_tau * (eq[0] - f[0]) - acc0);
 }
 
 // The same in the literal form, out of line (rarely taken).
 template <int LAT, int SCHEME, int VARIANT, bool FV>
 __device__ __noinline__ void cell_step_literal(const DevPlan& p, const unsigned* __restrict__ hf, int g,
-                                               const float* f0, const float* own, float ia, float* out) {
+                                               const float* f0, const float* own, float ia, float inv_tau, float dt,
+                                               float* out) {
   constexpr int NQ = Lat<LAT>::NQ;
   Slots<ResRows<LAT, SCHEME, VARIANT>::ROWS> s;
   load_rows(hf, g, s);
   float f[NQ], fn[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) f[q] = own[q];
-  cell_step<LAT, SCHEME, VARIANT, FV, true>(p, f0, s.w, ia, f, fn);
+  cell_step<LAT, SCHEME, VARIANT, FV, true>(p, f0, s.w, ia, inv_tau, dt, f, fn);
 #pragma unroll
   for (int q = 0; q < NQ; ++q) out[q] = fn[q];
 }
@@ -269,6 +270,13 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
   float* npdf = sm + size_t(2) * NQ * S;           // [max_nodes][NQ]
   float* sprod = npdf + size_t(NQ) * r.max_nodes;  // [max_st][SR]: macros and f - feq of the stencil cells
   const ResidentBlock b = r.block[blockIdx.x];
+  // a batch's case: its own constants; the blocks of a retired one only evaluate
+  // its nodes, once (no block imports from another case, and both buffers hold
+  // its final state)
+  const bool retired = p.case_active && !__ldg(p.case_active + b.cs);
+  if (retired) n_steps = 1;
+  const float inv_tau = p.case_active ? __ldg(p.case_inv_tau + b.cs) : p.inv_tau;
+  const float dt = p.case_active ? __ldg(p.case_dt + b.cs) : p.dt;
   // the block's node, ghost and import tables, read every step
   int4* t_nd = reinterpret_cast<int4*>(sm + (size_t(2) * NQ * S + size_t(NQ) * r.max_nodes + size_t(SR) * r.max_st + 3) / 4 * 4);
   float4* t_set = reinterpret_cast<float4*>(t_nd + b.nn);   // {sum of weights, set values, -}
@@ -486,7 +494,7 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
       uint4* ex = r.ex + size_t((s & 1) ^ 1) * NW * r.n_export;
       const int nf_own = *reinterpret_cast<volatile int*>(&s_nf[s % 3]);
       int nf_new = 0;
-      for (int l0 = ct & ~31; l0 < b.nown; l0 += TC) {
+      for (int l0 = ct & ~31; l0 < (retired ? 0 : b.nown); l0 += TC) {
         const int l = l0 + (tid & 31), g = b.own_off + l;
         if (!ONE) cls = __ldg(r.cls + (g >> 5));
         int nf = nf_own;
@@ -510,11 +518,11 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
             cell_step_fast<SCHEME>(p, f0, hold.w, f, fn);
           } else {
             if (nf) {
-              cell_step_literal<LAT, SCHEME, VARIANT, FV>(p, r.hf, g, f0, f0 + l * NQ, ia, f1 + l * NQ);
+              cell_step_literal<LAT, SCHEME, VARIANT, FV>(p, r.hf, g, f0, f0 + l * NQ, ia, inv_tau, dt, f1 + l * NQ);
 #pragma unroll
               for (int q = 0; q < NQ; ++q) fn[q] = f1[l * NQ + q];
             } else {
-              cell_step<LAT, SCHEME, VARIANT, FV, false>(p, f0, hold.w, ia, f, fn);
+              cell_step<LAT, SCHEME, VARIANT, FV, false>(p, f0, hold.w, ia, inv_tau, dt, f, fn);
             }
           }
           if (exp >= 0 && s + 1 < n_steps) {
@@ -542,6 +550,7 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
       if (s + 1 < n_steps) bar_arrive(2, T);
     }
   }
+  if (retired) return;
   __syncthreads();
 
   // the last two states, and the stencil macros of the last one

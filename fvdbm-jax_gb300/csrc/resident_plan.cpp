@@ -46,7 +46,7 @@ void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, s
 }  // namespace
 
 void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
-                    ResidentPlan& rp) {
+                    const float* case_dt, ResidentPlan& rp) {
   rp = ResidentPlan{};
   const int N = hp.N, H = hp.hrows;
   if (N == 0 || !hp.fusable || hp.K != 3 || n_blocks < 1) return;
@@ -69,8 +69,24 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     if (!std::isfinite(xy[i])) xy = nullptr;
   auto hfi = [&](int i, int row) { return size_t(i >> 5) * size_t(H) * 32 + size_t(row) * 32 + (i & 31); };
 
-  // ---- parts
-  const int B = std::min(n_blocks, N);
+  // ---- parts: those of a batch's case stay inside it, its share of the blocks
+  // by its cells (at least one; the cases with the most cells per block first)
+  const int B = std::min(n_blocks, N), S = std::max(1, hp.S);
+  if (S > B) return;
+  std::vector<int32_t> case_cell = hp.S ? hp.case_cell : std::vector<int32_t>{0, N}, share(S, 1);
+  for (int left = B - S; left > 0; --left) {
+    int best = -1;
+    double most = 1.0;
+    for (int s = 0; s < S; ++s) {
+      const double per = double(case_cell[s + 1] - case_cell[s]) / share[s];
+      if (per > most) {
+        most = per;
+        best = s;
+      }
+    }
+    if (best < 0) return;
+    ++share[best];
+  }
   std::vector<int32_t> ids(N), part_end(B), part(N), loc(N);
   {
     std::vector<Point> pts(N);
@@ -78,7 +94,8 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       const int32_t c = hp.cell_old[i];
       pts[i] = Point{{xy ? xy[2 * size_t(c)] : 0.0f, xy ? xy[2 * size_t(c) + 1] : 0.0f}, i};
     }
-    bisect(xy != nullptr, pts, 0, N, 0, B, part_end);
+    for (int s = 0, p0 = 0; s < S; p0 += share[s++])
+      bisect(xy != nullptr, pts, case_cell[s], case_cell[s + 1], p0, share[s], part_end);
     for (int i = 0; i < N; ++i) ids[i] = pts[i].id;
   }
   for (int t = 0, i = 0; t < B; ++t)
@@ -172,6 +189,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     ResidentBlock mb{};
     mb.own_off = off;
     mb.nown = b - a;
+    mb.cs = hp.S ? hp.cell_case[ids[a]] : 0;
     for (int i = a; i < b; ++i) {
       loc[ids[i]] = i - a;
       if (exported[ids[i]]) slot[ids[i]] = rp.n_export++;
@@ -266,7 +284,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
             const float D2 = f32(hp.hf[hfi(c, HR.d2(k))]);
             const float v[6] = {nx, ny, nx + ny, ny - nx, 2.0f * nx, 2.0f * ny};
             for (int j = 0; j < NP; ++j) {
-              const float t = (v[j] * pr.delta_t) / D2;
+              const float t = (v[j] * (case_dt ? case_dt[mb.cs] : pr.delta_t)) / D2;
               if (!std::isfinite(t)) finite_t = false;
               rp.hf[ri(g, 15 + 3 * j + k)] = bits(t);
             }

@@ -94,3 +94,28 @@ def test_non_finite_states(share, flux, lattice):
 @pytest.mark.parametrize("cells", [98, 3200, 120_000])
 def test_fast_family_runs_match_single_steps(cells, flux):
     _compare(_case(cells, flux), (4, 1, 20), "fast", "fast")
+
+
+@pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
+def test_batch_runs_match_single_steps(flux):
+    """Uneven cases with their own tau and dt, one of a few cells; one retires in
+    between and comes back."""
+    from fvdbm_jax_gb300 import Batch
+    cs = [_case(n, flux, seed=k) for k, n in enumerate((2, 98, 3200, 20_000, 800))]
+    for k, (c, _, _) in enumerate(cs):
+        c.dynamics.tau = 0.55 + 0.05 * k
+    a, b = Batch(cs), Batch(cs)
+    a.init()
+    b.init()
+    for n, active in ((5, None), (6, (1, 0, 1, 1, 1)), (1, None), (12, (1, 1, 0, 1, 0)), (5, (1, 1, 1, 1, 1))):
+        if active is not None:
+            a.set_active(active)
+            b.set_active(active)
+        a.step(n)
+        for _ in range(n):
+            b.step(1)
+        sa, sb = a.state(), b.state()
+        for k in sa:
+            assert np.array_equal(sa[k], sb[k], equal_nan=True), (n, k)
+    a.close()
+    b.close()
