@@ -25,8 +25,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-ffp-contract=off",
            "-I" + os.path.join(ROOT, "include")]
 SOURCES = ["kernels.cu", "tile.cu", "monitor.cu", "capi.cu", "plan.cpp", "batch.cpp", "mpnn.cu", "d2q13.cu",
-           "pcg.cu", "features.cu", "resident.cu", "resident_plan.cpp", "mpnn_layer.cu"]
-HEADERS = [os.path.join(CSRC, h) for h in ("fvdbm_internal.h", "fvdbm_math.cuh", "fvdbm_cell.cuh", "d2q13.cuh")] + [
+           "pcg.cu", "features.cu", "resident.cu", "resident_in_place.cu", "resident_plan.cpp", "mpnn_layer.cu"]
+HEADERS = [os.path.join(CSRC, h) for h in ("fvdbm_internal.h", "fvdbm_math.cuh", "fvdbm_cell.cuh", "d2q13.cuh", "resident.cuh")] + [
            os.path.join(ROOT, "include", "fvdbm.h"), os.path.join(ROOT, "include", "fvdbm_mpnn.h")]
 
 

@@ -28,6 +28,14 @@ constexpr int kGraphSteps = 32;  // steps per captured graph (even)
 // 16.1 / 15.2 and 10.9 / 7.6; 400k 15.8 / 17.0 at 4, 13.2 / 12.4 at 8, 10.7 /
 // 7.9 at 512.  A launch takes at most kResidentSteps.
 constexpr int kResidentMin = 4, kResidentMinLarge = 8;
+// Shared memory for two copies of the pdfs: at most this part of the chip's (the
+// rest: halos, tables); beyond it they move through a ring (resident_in_place.cu,
+// D2Q9 upwind), up to a part that leaves room for the ring's free chunk and
+// the boundary cells.  That pays from more steps on, us per step, per-step kernels / ring:
+// 425k cells 16.1 / 15.0 at 8 steps, 13.6 / 9.9 at 512; 480k 16.8 / 18.2 at 8,
+// 15.5 / 15.2 at 16, 14.2 / 12.4 at 512; contracted family, 480k, 13.0 / 12.7 at 16, 11.6 / 10.1.
+constexpr double kResidentPart = 0.85, kInPlacePart = 0.62;
+constexpr int kInPlaceMin = 16;
 constexpr int kLargeMesh = 1 << 18;  // cells from which AUTO takes the single-launch family
 constexpr int kResidentSteps = 1 << 20;
 constexpr int kResidentCells = 96;  // cells per block, at least (3.2k cells: 3.4 us per step, 3.9 at 128)
@@ -55,6 +63,7 @@ struct Handle {
   // resident step (resident.cu): runs of several steps in one launch, with the
   // state on the chip; res_tag: exchange tags used so far
   bool resident = false;
+  int res_min = 0;  // steps of a run, at least
   DevResident res{};
   size_t res_ex_bytes = 0;
   unsigned res_tag = 0;
@@ -272,10 +281,10 @@ int ensure_nodes(Handle* h) {
 
 constexpr int kPersistSteps = 4096;  // steps per cooperative launch, at most
 
-// A resident run may be queued: not while the stream is being captured (the
+// A resident run of n steps may be queued: not a short one, and not while the stream is being captured (the
 // exchange tags of a launch serve once, so it must not be replayed).
-bool resident_ready(Handle* h) {
-  if (!h->resident) return false;
+bool resident_ready(Handle* h, int n) {
+  if (!h->resident || n < h->res_min) return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
@@ -305,7 +314,7 @@ int run_resident(Handle* h, int n) {
 }
 
 int enqueue_steps(Handle* h, int n) {
-  if (h->persist && resident_ready(h)) return run_resident(h, n);
+  if (h->persist && resident_ready(h, n)) return run_resident(h, n);
   if (h->persist) {
     for (int done = 0; done < n;) {
       const int k = std::min(n - done, kPersistSteps);
@@ -409,13 +418,15 @@ std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh, co
   int sms = 0, lim = 0;
   const HostPlan& hp = h->hp;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess || hp.N == 0 ||
-      int64_t(hp.N) * 2 * hp.q * 4 > int64_t(sms) * lim)
+      cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess || hp.N == 0)
     return {};
+  const double chip = double(sms) * lim;
+  const bool in_place = double(hp.N) * 2 * hp.q * 4 > kResidentPart * chip;
+  if (in_place && (hp.q != 9 || hp.scheme != FVDBM_UPWIND || hp.variant != 0 || double(hp.N) * hp.q * 4 > kInPlacePart * chip)) return {};
   const int blocks = std::min(sms, (hp.N + kResidentCells - 1) / kResidentCells);
-  auto plan = [h, &mesh, blocks, case_dt] {
+  auto plan = [h, &mesh, blocks, case_dt, in_place] {
     ResidentPlan rp;
-    build_resident(mesh, h->params, h->hp, blocks, case_dt, rp);
+    build_resident(mesh, h->params, h->hp, blocks, case_dt, in_place, rp);
     return rp;
   };
   try {
@@ -437,7 +448,7 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   if (!rp.ok) return FVDBM_OK;
   DevResident& r = h->res;
   bool fits = false;
-  CK(prepare_resident(h->dp, rp, r, &fits));
+  CK(rp.in_place ? prepare_in_place(h->dp, rp, r, &fits) : prepare_resident(h->dp, rp, r, &fits));
   if (!fits) return FVDBM_OK;
   // one allocation and one copy for all tables
   std::vector<unsigned char> buf;
@@ -457,6 +468,7 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   put(r.halo_dev, rp.halo_dev);
   put(r.halo_exp, rp.halo_exp);
   put(r.st_loc, rp.st_loc);
+  put(r.halo_st, rp.halo_st);
   put(r.nd, rp.nd);
   put(r.nd_sw, rp.nd_sw);
   put(r.en_st, rp.en_st);
@@ -470,9 +482,12 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   const size_t words = size_t(2) * ((hp.q + 2) / 3) * size_t(std::max(rp.n_export, 1));
   if ((rc = dalloc<uint4>(h, &r.ex, words)) != FVDBM_OK) return rc;
   h->res_ex_bytes = words * sizeof(uint4);
+  if (rp.in_place && (rc = dalloc<float>(h, &r.rows, size_t(12) * rp.n_rows)) != FVDBM_OK) return rc;
   CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));
   CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
   h->resident = true;
+  // (the one cooperative launch of FVDBM_KERNEL_PERSIST costs as much)
+  h->res_min = rp.in_place ? kInPlaceMin : h->persist ? 1 : hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge;
   return FVDBM_OK;
 }
 
@@ -1192,7 +1207,7 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   if (mark) CK(cudaEventRecord(h->in_ready, h->stream));
   h->stepping = true;
   int n = n_steps;
-  if (n >= (h->hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge) && !h->persist && resident_ready(h)) {
+  if (!h->persist && resident_ready(h, n)) {
     int rc = run_resident(h, n);
     if (rc != FVDBM_OK) return rc;
     n = 0;

@@ -22,6 +22,7 @@ constexpr int Q = 9;
 constexpr int HF_SLOT1 = 1 << 2;
 constexpr int HF_GHOST = 1 << 3;
 constexpr int HF_SHIFT = 4;
+constexpr int IP_LINK = 20;  // in the update in place (resident_in_place.cu)
 constexpr int64_t HF_MAX_INDEX = (int64_t(1) << 27) - 1;
 
 // Persistent tile kernel: TILE consecutive cells per CTA iteration; the
@@ -171,12 +172,18 @@ struct ResidentBlock {
   int gh_off, ng;         // ghost entries of gh
   int last_st;            // stencil index of the cell that padded node entries read
   int en_off, ne;         // node entries of en_st / en_w
+  // the update in place: interior cells (the first of the own ones; the others
+  // start at the next multiple of 32), own cells among the stencil's
+  // (the first of them), rows kept of interior cells, the block's first row and
+  // export, cells of a chunk of the sweep
+  int nin, nst_own, nsave, row_off, exp_off, chunk;
   int cs;                 // the block's case (packed batch)
 };
 
 struct ResidentPlan {
-  bool ok = false;
+  bool ok = false, in_place = false;
   int n_export = 0;                    // exported cells of all blocks
+  int n_rows = 0;                      // in place: rows of all blocks
   int max_own = 0, stride = 0, max_nodes = 0, max_st = 0;
   int max_table = 0;                   // words of a block's tables in shared memory
   int cell_threads = 0, threads = 0;   // of a block (resident_threads)
@@ -188,6 +195,7 @@ struct ResidentPlan {
   std::vector<float> inv_area;
   std::vector<int32_t> halo_dev, halo_exp;
   std::vector<int32_t> st_loc;
+  std::vector<int32_t> halo_st;        // in place: a halo cell's stencil index (-1: none)
   std::vector<int32_t> nd;             // {device node, type | padded << 2 | owner << 3, first entry, entries}
   std::vector<float> nd_sw;
   std::vector<uint32_t> en_st;         // stencil index | ND_NEQ_ZERO
@@ -196,13 +204,14 @@ struct ResidentPlan {
   std::vector<int32_t> gh;             // {own cell, node a, node b, bits of the distance ratio}
 };
 void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
-                    const float* case_dt, ResidentPlan& rp);
+                    const float* case_dt, bool in_place, ResidentPlan& rp);
 void resident_threads(int max_own, int* cell_threads, int* threads);
+void in_place_threads(int max_in, int* cell_threads, int* threads);
 
 // Device view of the same; ex holds two buffers of ResidentPlan::n_export
 // cells, each cell as 16-byte words of three pdfs and the step's tag.
 struct DevResident {
-  int n_blocks, threads, cell_threads, n_export, stride, max_nodes, max_st;
+  int n_blocks, threads, cell_threads, n_export, stride, max_nodes, max_st, max_table;
   size_t smem;
   const void* kern;
   const ResidentBlock* block;
@@ -214,6 +223,7 @@ struct DevResident {
   const int* halo_dev;
   const int* halo_exp;
   const int* st_loc;
+  const int* halo_st;
   const int4* nd;
   const float* nd_sw;
   const unsigned* en_st;
@@ -221,6 +231,7 @@ struct DevResident {
   const int* fz_dev;
   const int4* gh;
   uint4* ex;
+  float* rows;  // in place: see there
 };
 
 // Build the plan; returns an empty string on success, else the reason.
@@ -359,8 +370,10 @@ cudaError_t launch_persist(const DevPlan& p, float* f0, float* f1, int n_steps, 
 // to p.node_*, and the stencil macros of f_last to p.cprod.  tag: the exchange
 // tags of the call's steps are tag + 1 .. tag + n_steps - 1 (never reused with
 // the same exchange buffer).  prepare_resident: threads and shared memory for the
-// plan, and whether the device can hold the grid.
+// plan, and whether the device can hold the grid.  prepare_in_place:
+// the same for a plan in place (resident_in_place.cu), which launch_resident launches too.
 cudaError_t prepare_resident(const DevPlan& p, const ResidentPlan& rp, DevResident& r, bool* fits);
+cudaError_t prepare_in_place(const DevPlan& p, const ResidentPlan& rp, DevResident& r, bool* fits);
 cudaError_t launch_resident(const DevPlan& p, const DevResident& r, const float* fin, float* f_prev, float* f_last,
                             int n_steps, unsigned tag, cudaStream_t s);
 // record the stencil macros of f (after an upload of the cell pdfs)

@@ -1,10 +1,13 @@
-// Host tables of the resident step (resident.cu): the cells are cut into
-// compact parts, one per thread block, and every index a block uses during a
-// run of steps becomes local to it: its own cells, then the halo cells it
-// imports from other blocks, then one ghost entry per ghost face.
+// Host tables of the resident steps: the cells are cut into compact parts, one
+// per thread block, and every index a block uses during a run of steps becomes
+// local to it: its own cells, then the halo cells it imports from other blocks,
+// then one ghost entry per ghost face (resident.cu); in place (resident_in_place.cu)
+// the interior cells in the order of the sweep, and rows for what the others read.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <future>
+#include <system_error>
 
 #include "fvdbm_internal.h"
 
@@ -39,15 +42,72 @@ void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, s
       return u.x[d] != v.x[d] ? u.x[d] < v.x[d] : u.id < v.id;
     });
   }
-  bisect(xy, pts, a, mid, p0, left, part_end);
+  std::future<void> other;  // (a large part's halves side by side)
+  try {
+    if (b - a > 1 << 16) other = std::async(std::launch::async, [&] { bisect(xy, pts, a, mid, p0, left, part_end); });
+  } catch (const std::system_error&) {
+  }
   bisect(xy, pts, mid, b, p0 + left, parts - left, part_end);
+  if (other.valid())
+    other.get();
+  else
+    bisect(xy, pts, a, mid, p0, left, part_end);
+}
+
+// Cells of a chunk of the sweep: chunks of equal size, at most a cell per thread.
+int chunk_cells(int inner, int threads) {
+  const int n = std::max(1, (inner + threads - 1) / threads);
+  return std::max(32, ((inner + n - 1) / n + 31) / 32 * 32);
+}
+
+// f(t) of every block, by a few threads (by fewer, or the caller, when there are
+// none to be had).
+template <class F>
+void for_blocks(int B, const F& f) {
+  constexpr int THREADS = 8;
+  std::vector<std::future<void>> work;
+  auto run = [&](int i) {
+    for (int t = i; t < B; t += THREADS) f(t);
+  };
+  for (int i = 0; i < THREADS && i < B; ++i) {
+    try {
+      work.push_back(std::async(std::launch::async, run, i));
+    } catch (const std::system_error&) {
+      run(i);
+    }
+  }
+  for (auto& w : work) w.get();
+}
+
+// Order of the update in place: the interior cells, the first `inner` of the
+// part's n, along the longer side of its bounding box, in chunks of TC.  Within
+// a chunk the device order (coalesced reads and writes of the state).
+void sweep_order(const float* xy, const HostPlan& hp, int32_t* ids, int n, int inner, int TC) {
+  if (!xy) return;
+  float lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
+  std::vector<Point> pts(n);
+  for (int i = 0; i < n; ++i) {
+    const size_t c = size_t(hp.cell_old[ids[i]]);
+    pts[i] = Point{{xy[2 * c], xy[2 * c + 1]}, ids[i]};
+    for (int d = 0; d < 2; ++d) {
+      lo[d] = std::min(lo[d], pts[i].x[d]);
+      hi[d] = std::max(hi[d], pts[i].x[d]);
+    }
+  }
+  const int d = hi[0] - lo[0] >= hi[1] - lo[1] ? 0 : 1;
+  std::sort(pts.begin(), pts.begin() + inner, [d](const Point& u, const Point& v) {
+    return u.x[d] != v.x[d] ? u.x[d] < v.x[d] : u.id < v.id;
+  });
+  for (int i = 0; i < inner; ++i) ids[i] = pts[i].id;
+  for (int i = 0; i < inner; i += TC) std::sort(ids + i, ids + std::min(inner, i + TC));
 }
 
 }  // namespace
 
 void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostPlan& hp, int n_blocks,
-                    const float* case_dt, ResidentPlan& rp) {
+                    const float* case_dt, bool in_place, ResidentPlan& rp) {
   rp = ResidentPlan{};
+  rp.in_place = in_place;
   const int N = hp.N, H = hp.hrows;
   if (N == 0 || !hp.fusable || hp.K != 3 || n_blocks < 1) return;
   // the kernel drops terms that are +-0 for finite geometry
@@ -64,6 +124,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   const bool lw = hp.scheme == FVDBM_LAX_WENDROFF, sc = hp.variant == FVDBM_VARIANT_FACE_SCALE;
   const int NP = hp.q == 13 ? 6 : 4;
   const int R = hp.fast ? H : 3 * ((lw ? 5 + NP : 4) + (sc ? 1 : 0));
+  if (in_place && (hp.q != 9 || lw || sc)) return;
   const float* xy = m.cell_xy;
   for (int64_t i = 0; xy && i < 2 * int64_t(N); ++i)
     if (!std::isfinite(xy[i])) xy = nullptr;
@@ -176,25 +237,41 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
         kind[c] = std::max<char>(kind[c], 1);
     }
   for (int t = 0; t < B; ++t) rp.max_own = std::max(rp.max_own, part_end[t] - (t ? part_end[t - 1] : 0));
-  resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
+  if (!in_place) resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
+  std::vector<int> inside(B);  // interior cells
+  for_blocks(B, [&](int t) {
+    const auto first = ids.begin() + (t ? part_end[t - 1] : 0), last = ids.begin() + part_end[t];
+    std::sort(first, last);
+    const auto in_end = std::stable_partition(first, last, [&](int32_t c) { return kind[c] == 0; });
+    std::stable_partition(in_end, last, [&](int32_t c) { return kind[c] == 1; });
+    inside[t] = int(in_end - first);
+  });
+  if (in_place) {
+    in_place_threads(*std::max_element(inside.begin(), inside.end()), &rp.cell_threads, &rp.threads);
+    for_blocks(B, [&](int t) {
+      const int a = t ? part_end[t - 1] : 0;
+      sweep_order(xy, hp, ids.data() + a, part_end[t] - a, inside[t], chunk_cells(inside[t], rp.cell_threads));
+    });
+  }
   int off = 0;
   for (int t = 0; t < B; ++t) {
     const int a = t ? part_end[t - 1] : 0, b = part_end[t];
-    std::sort(ids.begin() + a, ids.begin() + b);
-    const auto first = ids.begin() + a, last = ids.begin() + b;
-    const auto in_end = std::stable_partition(first, last, [&](int32_t c) { return kind[c] == 0; });
-    std::stable_partition(in_end, last, [&](int32_t c) { return kind[c] == 1; });
-    const int inner = int(in_end - first);
-    if (inner > rp.cell_threads) std::rotate(ids.begin() + a + rp.cell_threads, ids.begin() + a + inner, ids.begin() + b);
+    const int inner = inside[t], TC = rp.cell_threads;
+    if (!in_place && inner > TC) std::rotate(ids.begin() + a + TC, ids.begin() + a + inner, ids.begin() + b);
     ResidentBlock mb{};
     mb.own_off = off;
     mb.nown = b - a;
+    mb.nin = in_place ? inner : 0;
+    mb.exp_off = rp.n_export;
+    mb.chunk = chunk_cells(inner, TC);
     mb.cs = hp.S ? hp.cell_case[ids[a]] : 0;
+    // (the boundary cells of the update in place begin a group of 32)
+    const int gap = in_place ? (inner + 31) / 32 * 32 - inner : 0;
     for (int i = a; i < b; ++i) {
-      loc[ids[i]] = i - a;
+      loc[ids[i]] = i - a + (i - a < inner ? 0 : gap);
       if (exported[ids[i]]) slot[ids[i]] = rp.n_export++;
     }
-    off += (b - a + 31) / 32 * 32;
+    off += (b - a + gap + 31) / 32 * 32;
     rp.block.push_back(mb);
   }
   rp.dev.assign(off, -1);
@@ -211,17 +288,19 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   if (hp.fv) rp.inv_area.assign(off, 0.0f);
   std::vector<int32_t> hloc(N, -1), nloc(hp.M, -1), sloc(N, -1);
   std::vector<char> node_owned(hp.M, 0);
-  bool finite_t = true;
+  bool usable = true;
   for (int t = 0; t < B; ++t) {
     ResidentBlock& mb = rp.block[t];
     const int a = t ? part_end[t - 1] : 0, pad = (mb.nown + 31) / 32 * 32;
+    const int bnd0 = (mb.nin + 31) / 32 * 32, nb = mb.nown - mb.nin;
     std::sort(imp[t].begin(), imp[t].end(), [&](int32_t x, int32_t y) { return slot[x] < slot[y]; });
     mb.halo_off = int(rp.halo_dev.size());
     mb.nhalo = int(imp[t].size());
+    const int halo0 = in_place ? 0 : pad;
     for (int j = 0; j < mb.nhalo; ++j) {
       rp.halo_dev.push_back(imp[t][j]);
       rp.halo_exp.push_back(slot[imp[t][j]]);
-      hloc[imp[t][j]] = pad + j;
+      hloc[imp[t][j]] = halo0 + j;
     }
     auto local = [&](int32_t c) { return part[c] == t ? loc[c] : hloc[c]; };
     // boundary nodes: computed first, then frozen
@@ -232,6 +311,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     mb.last_st = 0;
     mb.en_off = int(rp.en_st.size());
     std::vector<int32_t> touched;
+    // (in place: the block's own ones first)
     auto st = [&](int32_t c) {
       if (sloc[c] < 0) {
         sloc[c] = mb.nst++;
@@ -240,6 +320,17 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       }
       return sloc[c];
     };
+    if (in_place) {
+      auto own = [&](int32_t c) {
+        if (part[c] == t) st(c);
+      };
+      for (int32_t d : nodes[t])
+        if (d < hp.Mc) {
+          if (hp.nd_npad[d] > 0) own(hp.last_cell_new);
+          for (int e = hp.nd_ptr[d]; e < hp.nd_ptr[d + 1]; ++e) own(int32_t(hp.nd_cell[e] & ~ND_NEQ_ZERO));
+        }
+      mb.nst_own = mb.nst;
+    }
     for (size_t j = 0; j < nodes[t].size(); ++j) {
       const int32_t d = nodes[t][j];
       nloc[d] = int(j);
@@ -262,13 +353,33 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
         rp.en_w.push_back(hp.nd_w[e]);
       }
     }
+    for (int j = 0; in_place && j < mb.nhalo; ++j) rp.halo_st.push_back(sloc[imp[t][j]]);
     for (int32_t c : touched) sloc[c] = -1;
     mb.ne = int(rp.en_st.size()) - mb.en_off;
-    // face slots with local indices; ghost faces get their own entries
+    // face slots with local indices; ghost faces get their own entries.  In
+    // place: the boundary cells' name rows, those of interior neighbours (saved)
+    // and of boundary cells after the ghosts
     mb.gh_off = int(rp.gh.size() / 4);
-    for (int l = 0; l < mb.nown; ++l) {
-      const int32_t c = ids[a + l];
-      const int g = mb.own_off + l;
+    int ng = 0;
+    for (int i = 0; in_place && i < mb.nown; ++i)
+      for (int k = 0; k < 3; ++k) {
+        const int32_t code = int32_t(hp.hf[hfi(ids[a + i], k)]);
+        if (code & HF_GHOST) ++ng;
+      }
+    std::vector<int32_t> saved(in_place ? mb.nin : 0, -1);
+    for (int i = mb.nin; in_place && i < mb.nown; ++i)
+      for (int k = 0; k < 3; ++k) {
+        const int32_t code = int32_t(hp.hf[hfi(ids[a + i], k)]), n = code >> HF_SHIFT;
+        if (!(code & HF_GHOST) && part[n] == t && loc[n] < mb.nin && saved[loc[n]] < 0)
+          saved[loc[n]] = mb.nsave++;
+      }
+    const int orow = mb.nhalo + ng, brow = orow + mb.nsave, ring = bnd0 + mb.chunk;
+    // (16 bits for a neighbour, 12 for a link)
+    if (in_place && (std::max(brow + nb, 9 * (ring + nb + 31)) > 0xffff || std::max(mb.nsave, nb) >= 0xfff)) usable = false;
+    for (int i = 0; i < mb.nown; ++i) {
+      const int32_t c = ids[a + i];
+      const int l = loc[c], g = mb.own_off + l;
+      const bool inside = i < mb.nin;
       rp.dev[g] = c;
       rp.exp[g] = slot[c];
       if (hp.fv) rp.inv_area[g] = hp.inv_area[c];
@@ -285,7 +396,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
             const float v[6] = {nx, ny, nx + ny, ny - nx, 2.0f * nx, 2.0f * ny};
             for (int j = 0; j < NP; ++j) {
               const float t = (v[j] * (case_dt ? case_dt[mb.cs] : pr.delta_t)) / D2;
-              if (!std::isfinite(t)) finite_t = false;
+              if (!std::isfinite(t)) usable = false;
               rp.hf[ri(g, 15 + 3 * j + k)] = bits(t);
             }
           }
@@ -298,21 +409,34 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
           const int gi = code >> HF_SHIFT;
           int32_t rbits;
           std::memcpy(&rbits, &hp.gh_r[gi], 4);
-          idx = pad + mb.nhalo + mb.ng++;
+          idx = (in_place ? mb.nhalo : pad + mb.nhalo) + mb.ng++;
           const int32_t row4[4] = {l, nloc[hp.gh_a[gi]], nloc[hp.gh_b[gi]], rbits};
           rp.gh.insert(rp.gh.end(), row4, row4 + 4);
         } else {
-          idx = local(code >> HF_SHIFT);
+          const int32_t n = code >> HF_SHIFT;
+          idx = local(n);
+          if (inside) {
+            // the sweep overwrites a chunk once the next one has been read
+            if (idx < mb.nin && std::abs(idx / mb.chunk - l / mb.chunk) > 1) usable = false;
+            idx = idx < mb.nin ? idx : ring + idx - bnd0;  // (the boundary cells follow the ring)
+            idx = (idx >> 5) * 288 + (idx & 31);
+          } else if (in_place && part[n] == t) {
+            idx = idx < mb.nin ? orow + saved[idx] : brow + idx - bnd0;
+          }
         }
-        rp.hf[ri(g, k)] = uint32_t((code & HF_SLOT1) | (idx << HF_SHIFT));
+        uint32_t link = 0;
+        if (in_place && k == 0) link = inside ? uint32_t(saved[i] + 1) : slot[c] < 0 ? 0u : uint32_t(slot[c] - mb.exp_off + 1);
+        rp.hf[ri(g, k)] = uint32_t((code & HF_SLOT1) | (idx << HF_SHIFT)) | link << IP_LINK;
       }
     }
-    rp.stride = std::max(rp.stride, pad + mb.nhalo + mb.ng);
+    mb.row_off = rp.n_rows;
+    rp.n_rows += orow + 2 * (mb.nsave + nb);
+    rp.stride = std::max(rp.stride, in_place ? bnd0 + mb.chunk + 2 * ((nb + 31) / 32 * 32) : pad + mb.nhalo + mb.ng);
     rp.max_nodes = std::max(rp.max_nodes, mb.nn + mb.nf);
     rp.max_st = std::max(rp.max_st, mb.nst);
-    rp.max_table = std::max(rp.max_table, 8 * mb.nn + 4 * mb.ng + 2 * mb.ne + mb.nst + mb.nhalo);
+    rp.max_table = std::max(rp.max_table, 8 * mb.nn + 4 * mb.ng + 2 * mb.ne + mb.nst + 2 * mb.nhalo);
   }
-  rp.ok = finite_t;
+  rp.ok = usable;
 }
 
 }  // namespace fvdbm

@@ -83,6 +83,39 @@ def test_many_cells_per_thread():
         _compare(_case(cells, "upwind"), (4, 1, 6), "auto", "fused")
 
 
+@pytest.mark.parametrize("cells,kernel,fv,special", [(420_000, "auto", False, 0.0), (430_000, "auto", True, 1e-6),
+                                                     (430_000, "fast", False, 0.0), (600_000, "auto", False, 0.0),
+                                                     (430_000, "persist", False, 0.0)])
+def test_in_place(cells, kernel, fv, special):
+    """From the capacity of two copies to that of the ring: two and more chunks,
+    runs that leave the ring at every offset."""
+    ref = "fast" if kernel == "fast" else "fused"
+    _compare(_case(cells, "upwind", special=special), (16, 1, 19), kernel, ref, fv=fv)
+
+
+def test_in_place_batch():
+    """Cases of one and of many blocks; one retires in between and comes back."""
+    from fvdbm_jax_gb300 import Batch
+    cs = [_case(n, "upwind", seed=k) for k, n in enumerate((2, 98, 3200, 200_000, 230_000))]
+    for k, (c, _, _) in enumerate(cs):
+        c.dynamics.tau = 0.55 + 0.05 * k
+    a, b = Batch(cs), Batch(cs)
+    a.init()
+    b.init()
+    for n, active in ((17, None), (16, (1, 0, 1, 0, 1)), (20, (1, 1, 1, 1, 1))):
+        if active is not None:
+            a.set_active(active)
+            b.set_active(active)
+        a.step(n)
+        for _ in range(n):
+            b.step(1)
+        sa, sb = a.state(), b.state()
+        for k in sa:
+            assert np.array_equal(sa[k], sb[k], equal_nan=True), (n, k)
+    a.close()
+    b.close()
+
+
 @pytest.mark.parametrize("lattice", ["D2Q9", "D2Q13"])
 @pytest.mark.parametrize("flux", ["upwind", "lax_wendroff"])
 @pytest.mark.parametrize("share", [1e-4, 2e-3])
