@@ -253,10 +253,10 @@ int upload_nodes(Handle* h) {
 }
 
 // Steps use programmatic dependent launch between the node and cell kernels
-// (each waits for its predecessor before it reads what one wrote; anything else
-// before a call's first launch, a copy or a kernel that does not trigger its
-// dependents, is waited for in full).  Single steps one call at a time, 3.2k cells: 8.0
-// us, 9.8 without it on the first launch.
+// (each waits for its predecessor before it reads what one wrote), the first
+// launch of a call when the call before was a step too: single steps, 3.2k
+// cells, 8.0 us, 9.8 without it.  After a copy or another kernel it gains
+// nothing (72 us for state in, step and state out, 74 with it).
 // The plan with the node pointers of buffer a (read) and b (written).
 DevPlan with_nodes(const Handle* h, int a, int b) {
   DevPlan q = h->dp;
@@ -313,7 +313,8 @@ int run_resident(Handle* h, int n) {
   return FVDBM_OK;
 }
 
-int enqueue_steps(Handle* h, int n) {
+// follows: the last work of the stream is a step.
+int enqueue_steps(Handle* h, int n, bool follows = false) {
   if (h->persist && resident_ready(h, n)) return run_resident(h, n);
   if (h->persist) {
     for (int done = 0; done < n;) {
@@ -331,6 +332,7 @@ int enqueue_steps(Handle* h, int n) {
   for (int s = 0; s < n; ++s) {
     const float* fin = h->f[h->cur];
     float* fout = h->f[h->cur ^ 1];
+    const bool pdl = s > 0 || follows;
     if (h->hp.q == 13) {
       if (h->fused)
         CK(launch13_fused(h->dp, fin, fout, h->stream));
@@ -341,8 +343,9 @@ int enqueue_steps(Handle* h, int n) {
       h->node_last = h->node_cur;
       h->node_cur ^= 1;
     } else if (h->batch) {
-      CK(launch_nodes(h->dp, fin, h->stream, /*pdl=*/true));
-      CK(launch_fused_batch(h->dp, fin, fout, h->stream, /*pdl=*/true, h->batch_block, h->batch_waves));
+      CK(launch_nodes(h->dp, fin, h->stream, pdl));
+      CK(launch_fused_batch(h->dp, fin, fout, h->stream, /*pdl=*/h->dp.NB > 0 || pdl, h->batch_block,
+                            h->batch_waves));
     } else if (h->one) {
       CK(launch_step(h->dp, fin, fout, h->stream, /*pdl=*/s > 0));
     } else if (h->tile) {
@@ -350,11 +353,11 @@ int enqueue_steps(Handle* h, int n) {
       CK(launch_tile(h->dp, fin, fout, h->stream));
     } else {
       if (h->fused)
-        CK(launch_nodes_cp(h->dp, fin, h->stream, /*pdl=*/true));
+        CK(launch_nodes_cp(h->dp, fin, h->stream, pdl));
       else
         CK(launch_nodes(h->dp, fin, h->stream, /*pdl=*/s > 0));
       if (h->fused) {
-        CK(launch_fused(h->dp, fin, fout, h->stream, /*pdl=*/true));
+        CK(launch_fused(h->dp, fin, fout, h->stream, /*pdl=*/h->dp.NB > 0 || pdl));
       } else {
         CK(launch_face_flux(h->dp, fin, h->flux, h->stream));
         CK(launch_gather(h->dp, fin, h->flux, fout, h->stream));
@@ -450,7 +453,7 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   bool fits = false;
   CK(rp.in_place ? prepare_in_place(h->dp, rp, r, &fits) : prepare_resident(h->dp, rp, r, &fits));
   if (!fits) return FVDBM_OK;
-  // one allocation and one copy for all tables
+  // one allocation for all, one copy for the tables
   std::vector<unsigned char> buf;
   std::vector<std::pair<const void**, size_t>> at;  // field, offset
   auto put = [&](auto& field, const auto& vec) {
@@ -475,14 +478,15 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   put(r.en_w, rp.en_w);
   put(r.fz_dev, rp.fz_dev);
   put(r.gh, rp.gh);
+  const size_t ex_at = (buf.size() + 255) / 256 * 256;
+  h->res_ex_bytes = size_t(2) * ((hp.q + 2) / 3) * size_t(std::max(rp.n_export, 1)) * sizeof(uint4);
+  const size_t rows_at = ex_at + (h->res_ex_bytes + 255) / 256 * 256;
   unsigned char* base = nullptr;
-  int rc = dalloc(h, &base, buf.size(), &buf);
+  int rc = dalloc(h, &base, rows_at + size_t(12) * rp.n_rows * sizeof(float), &buf);
   if (rc != FVDBM_OK) return rc;
   for (auto& a : at) *a.first = base + a.second;
-  const size_t words = size_t(2) * ((hp.q + 2) / 3) * size_t(std::max(rp.n_export, 1));
-  if ((rc = dalloc<uint4>(h, &r.ex, words)) != FVDBM_OK) return rc;
-  h->res_ex_bytes = words * sizeof(uint4);
-  if (rp.in_place && (rc = dalloc<float>(h, &r.rows, size_t(12) * rp.n_rows)) != FVDBM_OK) return rc;
+  r.ex = reinterpret_cast<uint4*>(base + ex_at);
+  r.rows = reinterpret_cast<float*>(base + rows_at);
   CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));
   CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
   h->resident = true;
@@ -1205,6 +1209,7 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   // follow another one is marked for the read-back beside it)
   const bool mark = n_steps == 1 && h->hp.N > 0 && !h->stepping;
   if (mark) CK(cudaEventRecord(h->in_ready, h->stream));
+  const bool follows = h->stepping;
   h->stepping = true;
   int n = n_steps;
   if (!h->persist && resident_ready(h, n)) {
@@ -1224,7 +1229,7 @@ int fvdbm_step(void* handle, int32_t n_steps) {
       if (h->fnodes) h->node_last = h->node_cur ^ 1;
     }
   }
-  int rc = enqueue_steps(h, n);
+  int rc = enqueue_steps(h, n, follows);
   if (rc != FVDBM_OK) return rc;
   h->in_ok = mark;
   h->steps_done += n_steps;

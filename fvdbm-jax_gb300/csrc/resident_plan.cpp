@@ -15,6 +15,8 @@ namespace fvdbm {
 
 namespace {
 
+constexpr int MANY = 1 << 16;  // cells from which threads pay
+
 struct Point {
   float x[2];
   int32_t id;
@@ -44,7 +46,7 @@ void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, s
   }
   std::future<void> other;  // (a large part's halves side by side)
   try {
-    if (b - a > 1 << 16) other = std::async(std::launch::async, [&] { bisect(xy, pts, a, mid, p0, left, part_end); });
+    if (b - a > MANY) other = std::async(std::launch::async, [&] { bisect(xy, pts, a, mid, p0, left, part_end); });
   } catch (const std::system_error&) {
   }
   bisect(xy, pts, mid, b, p0 + left, parts - left, part_end);
@@ -60,10 +62,14 @@ int chunk_cells(int inner, int threads) {
   return std::max(32, ((inner + n - 1) / n + 31) / 32 * 32);
 }
 
-// f(t) of every block, by a few threads (by fewer, or the caller, when there are
-// none to be had).
+// f(t) of every block, by a few threads for a large mesh of N cells (by fewer, or
+// the caller, when there are none to be had).
 template <class F>
-void for_blocks(int B, const F& f) {
+void for_blocks(int N, int B, const F& f) {
+  if (N < MANY) {
+    for (int t = 0; t < B; ++t) f(t);
+    return;
+  }
   constexpr int THREADS = 8;
   std::vector<std::future<void>> work;
   auto run = [&](int i) {
@@ -239,7 +245,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   for (int t = 0; t < B; ++t) rp.max_own = std::max(rp.max_own, part_end[t] - (t ? part_end[t - 1] : 0));
   if (!in_place) resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
   std::vector<int> inside(B);  // interior cells
-  for_blocks(B, [&](int t) {
+  for_blocks(N, B, [&](int t) {
     const auto first = ids.begin() + (t ? part_end[t - 1] : 0), last = ids.begin() + part_end[t];
     std::sort(first, last);
     const auto in_end = std::stable_partition(first, last, [&](int32_t c) { return kind[c] == 0; });
@@ -248,7 +254,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   });
   if (in_place) {
     in_place_threads(*std::max_element(inside.begin(), inside.end()), &rp.cell_threads, &rp.threads);
-    for_blocks(B, [&](int t) {
+    for_blocks(N, B, [&](int t) {
       const int a = t ? part_end[t - 1] : 0;
       sweep_order(xy, hp, ids.data() + a, part_end[t] - a, inside[t], chunk_cells(inside[t], rp.cell_threads));
     });
