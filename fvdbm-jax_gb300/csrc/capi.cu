@@ -21,21 +21,21 @@ std::mutex g_err_mu;
 std::string g_create_err;
 
 constexpr int kGraphSteps = 32;  // steps per captured graph (even)
-// Runs of at least this many steps go to the resident kernel, when the state
-// fits on the chip: its launch loads and stores the whole state (about 20 us
-// with the launch), which a short run does not win back.  us per step, per-step
-// kernels / resident: 60k cells 13.0 / 9.9 at 4 steps, 8.2 / 3.2 at 512; 250k
-// 16.1 / 15.2 and 10.9 / 7.6; 400k 15.8 / 17.0 at 4, 13.2 / 12.4 at 8, 10.7 /
-// 7.9 at 512.  A launch takes at most kResidentSteps.
-constexpr int kResidentMin = 4, kResidentMinLarge = 8;
-// Shared memory for two copies of the pdfs: at most this part of the chip's (the
-// rest: halos, tables); beyond it they move through a ring (resident_in_place.cu,
-// D2Q9 upwind), up to a part that leaves room for the ring's free chunk and
-// the boundary cells.  That pays from more steps on, us per step, per-step kernels / ring:
-// 425k cells 16.1 / 15.0 at 8 steps, 13.6 / 9.9 at 512; 480k 16.8 / 18.2 at 8,
-// 15.5 / 15.2 at 16, 14.2 / 12.4 at 512; contracted family, 480k, 13.0 / 12.7 at 16, 11.6 / 10.1.
-constexpr double kResidentPart = 0.85, kInPlacePart = 0.62;
-constexpr int kInPlaceMin = 16;
+// Runs of several steps go to a resident kernel, when the state fits on the
+// chip: with two copies of the pdfs (resident.cu) up to kResidentPart of its shared memory
+// (the rest: halos, tables), or D2Q9 upwind through a ring (resident_in_place.cu)
+// up to a part that leaves room for the ring's free chunk and the
+// boundary cells.  The ring's two halves of a block's warps work side by side, but
+// wait for each other once a step; us per step, two copies / ring (porous):
+// 130k cells 4.9 / 5.4, 180k 5.5 / 5.6, 250k 7.7 / 6.6, 320k 8.9 / 7.5; contracted
+// family 180k 4.7 / 5.3, 250k 6.7 / 6.1.
+constexpr double kResidentPart = 0.85, kRingPart = 0.42, kInPlacePart = 0.62;
+// The steps of a run, at least: a launch loads and stores the whole state.  us per
+// step, per-step kernels / resident: 60k cells 13.0 / 9.9 at 4 steps, 8.2 / 3.2 at 512; 250k 16.9 / 13.8
+// at 4, 12.1 / 6.9 at 64; 300k 16.9 / 16.8 at 4, 14.6 / 12.2 at 8; 400k 17.8 / 20.2
+// at 4, 15.7 / 15.0 at 8, 13.5 / 10.4 at 64; 480k 15.8 / 16.1 at 12, 15.5 / 15.2 at
+// 16, 14.2 / 12.4 at 512.  A launch takes at most kResidentSteps.
+constexpr int kResidentMin = 4, kResidentMinLarge = 8, kResidentMinRing = 16;
 constexpr int kLargeMesh = 1 << 18;  // cells from which AUTO takes the single-launch family
 constexpr int kResidentSteps = 1 << 20;
 constexpr int kResidentCells = 96;  // cells per block, at least (3.2k cells: 3.4 us per step, 3.9 at 128)
@@ -424,12 +424,17 @@ std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh, co
       cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess || hp.N == 0)
     return {};
   const double chip = double(sms) * lim;
-  const bool in_place = double(hp.N) * 2 * hp.q * 4 > kResidentPart * chip;
-  if (in_place && (hp.q != 9 || hp.scheme != FVDBM_UPWIND || hp.variant != 0 || double(hp.N) * hp.q * 4 > kInPlacePart * chip)) return {};
+  const bool twice = double(hp.N) * 2 * hp.q * 4 <= kResidentPart * chip;
+  const bool ring = hp.q == 9 && hp.scheme == FVDBM_UPWIND && hp.variant == 0 &&
+                    double(hp.N) * 2 * hp.q * 4 > kRingPart * chip && double(hp.N) * hp.q * 4 <= kInPlacePart * chip;
+  if (!twice && !ring) return {};
+  // (the one cooperative launch of FVDBM_KERNEL_PERSIST costs as much)
+  h->res_min = !twice ? kResidentMinRing : h->persist ? 1 : hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge;
   const int blocks = std::min(sms, (hp.N + kResidentCells - 1) / kResidentCells);
-  auto plan = [h, &mesh, blocks, case_dt, in_place] {
+  auto plan = [h, &mesh, blocks, case_dt, twice, ring] {
     ResidentPlan rp;
-    build_resident(mesh, h->params, h->hp, blocks, case_dt, in_place, rp);
+    if (ring) build_resident(mesh, h->params, h->hp, blocks, case_dt, true, rp);
+    if (!rp.ok && twice) build_resident(mesh, h->params, h->hp, blocks, case_dt, false, rp);
     return rp;
   };
   try {
@@ -490,8 +495,6 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));
   CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
   h->resident = true;
-  // (the one cooperative launch of FVDBM_KERNEL_PERSIST costs as much)
-  h->res_min = rp.in_place ? kInPlaceMin : h->persist ? 1 : hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge;
   return FVDBM_OK;
 }
 

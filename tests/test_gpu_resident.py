@@ -83,14 +83,45 @@ def test_many_cells_per_thread():
         _compare(_case(cells, "upwind"), (4, 1, 6), "auto", "fused")
 
 
-@pytest.mark.parametrize("cells,kernel,fv,special", [(420_000, "auto", False, 0.0), (430_000, "auto", True, 1e-6),
+@pytest.mark.parametrize("cells,kernel,fv,special", [(215_000, "auto", False, 0.0), (250_000, "auto", True, 1e-6),
+                                                     (300_000, "fast", False, 0.0), (420_000, "auto", True, 0.0),
                                                      (430_000, "fast", False, 0.0), (600_000, "auto", False, 0.0),
                                                      (430_000, "persist", False, 0.0)])
 def test_in_place(cells, kernel, fv, special):
-    """From the capacity of two copies to that of the ring: two and more chunks,
-    runs that leave the ring at every offset."""
+    """From the line where the ring is faster to its capacity: two and more
+    chunks, runs that leave the ring at every offset."""
     ref = "fast" if kernel == "fast" else "fused"
     _compare(_case(cells, "upwind", special=special), (16, 1, 19), kernel, ref, fv=fv)
+
+
+def test_two_copies_near_capacity():
+    """What the ring does not take."""
+    _compare(_case(400_000, "lax_wendroff"), (8, 9), "auto", "fused")
+    _compare(_case(270_000, "upwind", lattice="D2Q13"), (8, 9), "auto", "fused")
+
+
+def test_ring_without_coordinates():
+    """The sweep's order needs them: the device order, or two copies."""
+    import ctypes as C
+
+    from fvdbm_jax_gb300 import _native as nat
+    from fvdbm_jax_gb300.environment import pack
+    cfn = _case(220_000, "upwind")
+    pdf = np.ascontiguousarray(cfn[0].pdf, np.float32)
+    out = []
+    for runs in ((17,), (1,) * 17):
+        mesh, params, keep, *_ = pack(*cfn, kernel="auto")
+        mesh.cell_xy = None
+        L, h = nat.lib(), C.c_void_p()
+        nat.check(L.fvdbm_create(C.byref(mesh), C.byref(params), C.byref(h)), None)
+        nat.check(L.fvdbm_set_state(h, nat.fptr(pdf), None, None, None), h)
+        for n in runs:
+            nat.check(L.fvdbm_step(h, n), h)
+        got = np.empty_like(pdf)
+        nat.check(L.fvdbm_get_cells(h, nat.fptr(got), None, None, None), h)
+        L.fvdbm_destroy(h)
+        out.append(got)
+    assert np.array_equal(*out)
 
 
 def test_in_place_batch():
