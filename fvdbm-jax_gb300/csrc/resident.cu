@@ -23,7 +23,8 @@
 // boundary, about 6,500 clocks; beyond, the cell warps' issue and shared-memory
 // slots.  us per step, best per-step family before / now (runs of 512
 // steps): 3.2k cells 7.2 / 3.1, 60k upwind 8.2 / 3.2, 60k Lax-Wendroff 10.2 /
-// 3.4, 60k D2Q13 14.2 / 4.9, 250k 10.9 / 7.6, 400k 10.7 / 7.9.  One barrier for
+// 3.4, 60k D2Q13 14.2 / 4.9, 250k 10.9 / 7.6, 400k 10.7 / 7.9 (D2Q9 upwind takes
+// resident_in_place.cu from 206k on).  One barrier for
 // all warps and the nodes in line with the cells measured 3.4, 4.5, 5.7, 6.8,
 // 10.4 and 11.5; row-wise tables read through L1 each step 3.3, 3.3, 3.5, 4.9, 8.4
 // and 8.7.

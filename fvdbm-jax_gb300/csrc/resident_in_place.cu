@@ -1,5 +1,6 @@
-// The resident step for meshes whose state fits on the chip once, but not twice
-// (resident.cu): a block's interior pdfs move through a ring in shared memory.
+// The resident step for meshes of many cells per block, whose state need not fit on
+// the chip twice (resident.cu): a block's interior pdfs move through a ring in
+// shared memory.
 //
 // A step in each block, one per SM, its two halves side by side:
 //   cell warps   sweep the interior cells (whose neighbours are all the block's
@@ -15,11 +16,12 @@
 //
 // Rows are the block's own scratch in global memory (L1 and L2).
 //
-// Bound by latency: the sweep takes about 3,200 clocks per chunk of 512 cells
-// (525 instructions per cell on 16 warps), the aux warps' chain of rounds through the
-// halo import about 18,000; both run at once.  us per step, the two launches of a step /
-// here: porous, 425k cells 13.6 / 9.9, contracted family 11.4 / 8.7; 24 cases of
-// 422k cells in all 22 / 15.
+// Bound by latency, at 425k cells: the sweep takes about 3,200 clocks per chunk of 512
+// cells (525 instructions per cell on 16 warps), the aux warps' chain of rounds
+// through the halo import about 18,000; both run at once.  us per step, one or two
+// launches of a step / here: porous, 250k cells 12.1 / 6.6, 425k 13.6 / 9.9, contracted
+// family 11.1 / 6.1 and 11.4 / 8.7; 24 cases of 422k cells in all 22 / 15.  Boundary
+// cells after the sweep, by the cell warps: 11.1 and 8.8 at 425k.
 #include "resident.cuh"
 
 namespace fvdbm {
@@ -27,8 +29,8 @@ namespace fvdbm {
 namespace {
 
 constexpr int IP_THREADS = 1024;
-constexpr int IP_ROW = 12;       // floats of a row: q = 1..8, 0, and padding
-constexpr int IP_SR = 12;        // floats of a stencil cell: macros, f - feq
+constexpr int IP_ROW = 12;  // floats of a row: q = 1..8, 0, and padding
+constexpr int IP_SR = 12;   // floats of a stencil cell: macros, f - feq
 
 // A face's code: HF_SLOT1, the neighbour (16 bits from HF_SHIFT); in the first
 // one, from bit IP_LINK on, 1 + the row of an interior cell that boundary cells

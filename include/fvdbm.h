@@ -64,9 +64,10 @@ extern "C" {
                                      FUSED below and for D2Q13, STAGED when the fused kernels
                                      cannot run: not triangles, padded or foreign face slots,
                                      per-q flux scale).  Runs of several steps (fvdbm_step with
-                                     n_steps >= 8) of a mesh whose state fits on the chip (about
-                                     400,000 D2Q9 triangles) take one launch, with the same
-                                     results; FAST does too */
+                                     n_steps >= 4, 8 or 16 by size) of a mesh whose state fits on
+                                     the chip (D2Q9 about 400,000 triangles, upwind about 600,000)
+                                     take one launch, with the same results; FAST and packed
+                                     batches do too */
 #define FVDBM_KERNEL_STAGED 1     /* node BC + face flux + cell gather (3 kernels) */
 #define FVDBM_KERNEL_FUSED 2      /* node BC + fused cell kernel (2 kernels; triangles) */
 #define FVDBM_KERNEL_TILE 3       /* persistent tile kernel, nodes evaluated in-tile (1 kernel) */
@@ -279,7 +280,8 @@ int fvdbm_run_to_steady(void *handle, double threshold, int32_t check_every, int
  * Environment at a time).  n_cases independent cases in one handle: their
  * meshes are joined into one device mesh (cells of a case stay contiguous,
  * ordered within the case), so each step is one node launch and one cell
- * launch for all cases, with each case's own 1/tau and delta_t.  Every case
+ * launch for all cases (one launch for a run of steps when they fit on the
+ * chip), with each case's own 1/tau and delta_t.  Every case
  * evolves bit for bit as it would in its own handle.  Cases that converge
  * retire: their cells are no longer read or written.  Needs triangles (3
  * face slots per cell) and no flux-scale variant; params[s] may differ only in
