@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(BR) k_bin_rows(int n, int nbins, const int* __
     }
     pos += all;
   }
-  for (int c = b * BR + int(threadIdx.x); c < n; c += nbins * BR) ucol[c] = bin_off + bin[c];
+  for (size_t c = size_t(b) * BR + threadIdx.x; c < size_t(n); c += size_t(nbins) * BR) ucol[c] = bin_off + bin[c];
 }
 
 }  // namespace

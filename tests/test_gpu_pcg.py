@@ -135,7 +135,7 @@ def test_pcg_sizes(n):
 
 
 @pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 5000])
-@pytest.mark.parametrize("bins", [1, 16, 300])
+@pytest.mark.parametrize("bins", [1, 16, 300, (1 << 21) + 1])
 def test_bin_rows(n, bins):
     """Each bin's cells in ascending order, against a stable sort by bin."""
     import torch
