@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(TCW * 32) k_dense_tc(const float* __restrict__
                                                        const float* __restrict__ residual, float* __restrict__ z,
                                                        float* __restrict__ ya, int split, int acc_a,
                                                        float* __restrict__ yb) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int K = da + db;
   const int Kp = (K + 7) & ~7, Op = (dout + 7) & ~7;
   const int ws = Op + 8, xsd = Kp + 4;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(TCW * 32) k_dense_wgrad_tc(const float* __rest
                                                             const float* __restrict__ xa, int da,
                                                             const float* __restrict__ xb, int db, int chunk,
                                                             float* __restrict__ part) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int K = da + db;
   const int Mp = (dout + 15) & ~15, Np = (K + 1 + 7) & ~7;
   const int zsd = Mp + 4, xsd = Np + 8;
@@ -407,7 +407,7 @@ constexpr int LRC = 128, LRF = 64;  // chunks per stage, features per block
 __global__ void __launch_bounds__(512) k_spmm_long_rows(const int* __restrict__ chunk_ptr, int n,
                                                         const float* __restrict__ partial, int d,
                                                         float* __restrict__ out, int accumulate) {
-  extern __shared__ float st[];  // [2][LRC][LRF]
+  extern __shared__ __align__(16) float st[];  // [2][LRC][LRF]
   __shared__ int list[512], count;
   const int f0 = blockIdx.y * LRF, nf = min(LRF, d - f0), tid = threadIdx.x;
   const bool vec = nf == LRF && d % 4 == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0;

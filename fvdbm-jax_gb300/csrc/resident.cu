@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
   using L = Lat<LAT>;
   constexpr int NQ = L::NQ, NW = (NQ + 2) / 3, SR = NQ + 4;  // SR: row of sprod (odd)
   constexpr int ROWS = FAST ? HfFastRows{3, SCHEME}.rows() : ResRows<LAT, SCHEME, VARIANT>::ROWS;
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   __shared__ unsigned long long s_bar[2];  // halo imported, ghosts evaluated
   __shared__ int s_bad;                    // 1 + step of a failed wait
   __shared__ int s_nf[3], s_nfx[3];        // a pdf of state s % 3 is not finite: own cells; halo or ghosts
