@@ -168,12 +168,15 @@ __global__ void __launch_bounds__(ONE ? 640 : 1024, 1)
         if (nf) s_nfx[s % 3] = 1;
       }
       // the own cells of this state are complete, and no cell warp still
-      // waits for the previous step's phase
-      if (s > 0) bar_sync(2, T);
-      if (at == 0) {
-        s_nfx[(s + 1) % 3] = 0;
-        mbar_arrive(bar_halo);
+      // waits for the previous step's phase.  The flag of state s + 1 is cleared
+      // before the barrier (state 1's starts clear): a warp sets it while it imports
+      // that state, which in a block without nodes and ghosts it may do right after the
+      // barrier.  The cell warps read it last for state s - 2, two barriers ago.
+      if (s > 0) {
+        if (at == 0) s_nfx[(s + 1) % 3] = 0;
+        bar_sync(2, T);
       }
+      if (at == 0) mbar_arrive(bar_halo);
       if (b.nn > 0) {
         // macros and f - feq of the stencil cells
         for (int j = at; j < b.nst; j += TA) {
