@@ -65,7 +65,7 @@ EXPORTS = ["fvdbm_create", "fvdbm_set_state", "fvdbm_step", "fvdbm_step_phase", 
            "fvdbm_batch_run_to_steady_time", "fvdbm_batch_residual_cases",
            "fvdbm_mp_dense_fwd", "fvdbm_mp_dense_bwd_data", "fvdbm_mp_wgrad_scratch", "fvdbm_mp_dense_bwd_weight",
            "fvdbm_mp_relu_bwd", "fvdbm_mp_spmm", "fvdbm_mp_mse_scratch", "fvdbm_mp_mse", "fvdbm_mp_adam",
-           "fvdbm_mp_to_bf16", "fvdbm_mp_spmm_chunked", "fvdbm_pcg_work_bytes", "fvdbm_pcg",
+           "fvdbm_mp_to_bf16", "fvdbm_mp_spmm_chunked", "fvdbm_pcg_work_bytes", "fvdbm_pcg", "fvdbm_pcg_bounded",
            "fvdbm_ws_wall_distance", "fvdbm_ws_potential_rows", "fvdbm_ws_potential_grad", "fvdbm_ws_mesh_mean",
            "fvdbm_ws_bin_ids", "fvdbm_ws_bin_rows", "fvdbm_mp_fused_scratch", "fvdbm_mp_layer_fwd",
            "fvdbm_mp_layer_bwd", "fvdbm_mp_enc_fwd", "fvdbm_mp_enc_bwd", "fvdbm_mp_dec_fwd", "fvdbm_mp_dec_bwd"]
@@ -130,6 +130,7 @@ def lib(build_if_missing: bool = True) -> C.CDLL:
     L.fvdbm_pcg_work_bytes.restype = sz
     L.fvdbm_pcg.argtypes = [i32, u64, u64, u64, u64, u64, i32, C.c_double, i32, u64, sz, u64,
                             C.POINTER(C.c_int32), C.POINTER(C.c_double)]
+    L.fvdbm_pcg_bounded.argtypes = L.fvdbm_pcg.argtypes[:9] + [i32] + L.fvdbm_pcg.argtypes[9:]
     L.fvdbm_ws_wall_distance.argtypes = [i32, u64, u64, i32, u64, u64, u64, u64]
     L.fvdbm_ws_potential_rows.argtypes = [i32, u64, u64, u64, u64, u64, u64, i32, u64, u64, u64, u64]
     L.fvdbm_ws_potential_grad.argtypes = [i32, u64, u64, u64, u64, u64, u64, u64, u64, u64, u64, u64, u64, u64]

@@ -172,10 +172,11 @@ __global__ void __launch_bounds__(PT) k_direction(int n, const double* __restric
 // its groups as 16-byte words {double, tag}, each one 128-bit access, and
 // every block collects all of them.  Sums run in the order of the kernels above
 // (group partials by the same tree, then k_scalars' order), so the iterates
-// are the same bits.  Waits are bounded: one that runs out sets *fail and ends
-// the launch.
+// are the same bits.  Waits are bounded (other work on the GPU may keep a block
+// from starting): one that runs out sets *fail and ends the launch, whose solution
+// is then not taken (it waits in the rows' words) and the kernels above solve the system.
 constexpr int PV = 4;                  // row groups a block works on side by side (PV * PT threads)
-constexpr int PCG_POLLS = 1 << 20;
+constexpr int PCG_POLLS = 1 << 20;     // of one wait (about a second)
 
 __device__ __forceinline__ bool get_word(const uint4* ptr, unsigned tag, double* v) {
   unsigned long long a, b;
@@ -188,8 +189,8 @@ __device__ __forceinline__ bool get_word(const uint4* ptr, unsigned tag, double*
   return unsigned(b) == tag && unsigned(b >> 32) == tag;
 }
 // Waits for the row's word of iteration `tag` (bounded).
-__device__ __forceinline__ bool get_row(const uint4* ptr, unsigned tag, float* z, float* p) {
-  for (int it = 0; it < PCG_POLLS; ++it) {
+__device__ __forceinline__ bool get_row(const uint4* ptr, unsigned tag, int polls, float* z, float* p) {
+  for (int it = 0; it < polls; ++it) {
     double v;
     if (get_word(ptr, tag, &v)) {
       const unsigned long long a = (unsigned long long)__double_as_longlong(v);
@@ -211,12 +212,11 @@ __device__ __forceinline__ void put_row(uint4* ptr, unsigned tag, float z, float
 }
 
 struct SolveArgs {
-  int n, groups, per_block, max_iter, check_every;
+  int n, groups, per_block, max_iter, check_every, polls;
   double rtol;
   const int *ip, *ix;
-  const float *v, *b;
-  float* x;
-  uint4* zp;    // [n]: {z, p of the iteration before, tag, tag}
+  const float *v, *b, *x;
+  uint4* zp;    // [n]: {z, p of the iteration before, tag, tag}; out: {x, -, -, -}
   uint4* ex;    // [2][3][groups]: the exchange words of even and odd exchanges
   double* s;    // out: S_RZ, S_RR, S_BB
   int* fail;    // out: {a wait ran out, iterations}
@@ -265,13 +265,14 @@ __device__ __forceinline__ bool exchange(const SolveArgs& a, double (*part)[3], 
                                          double* d, double rz, double* tot, int* s_ok) {
   constexpr int NWD = 4;  // words per thread, at most: 3 * 1216 groups over 1024 threads
   __shared__ double s_tot[4];
+  __shared__ int s_go;
   __syncthreads();
   uint4* ex = a.ex + size_t(tag & 1) * 3 * a.groups;
   const int tid = threadIdx.x, nt = blockDim.x, words = K * a.groups;
   if (tid < ng * K) put_word(ex + size_t(tid % K) * a.groups + g0 + tid / K, tag, part[tid / K][tid % K]);
   double v[NWD];
   bool all = false;
-  for (int it = 0; it < PCG_POLLS && !all; ++it) {
+  for (int it = 0; it < a.polls && !all; ++it) {
     all = true;
 #pragma unroll
     for (int i = 0; i < NWD; ++i)
@@ -300,13 +301,14 @@ __device__ __forceinline__ bool exchange(const SolveArgs& a, double (*part)[3], 
       // (one thread divides: 1024 would take 7,000 clocks)
       if (tid == 0 && K == 1) s_tot[1] = s != 0.0 ? rz / s : 0.0;
       if (tid == 0 && K == 2) s_tot[2] = rz != 0.0 ? s / rz : 0.0;
+      if (tid == 0) s_go = *s_ok;  // (one answer for the block: a thread that is ahead may clear *s_ok again)
     }
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k <= (K < 3 ? K : 2); ++k) tot[k] = s_tot[k];
-  if (!*s_ok && tid == 0) atomicExch(a.fail, 1);
-  return *s_ok != 0;
+  if (!s_go && tid == 0) atomicExch(a.fail, 1);
+  return s_go != 0;
 }
 
 template <int R>
@@ -398,7 +400,7 @@ __global__ void __launch_bounds__(PV* PT, 1) k_solve(SolveArgs a) {
       // direction of row c
       auto dir = [&](int c) {
         float zc = 0.0f, pc = 0.0f;
-        if (!get_row(a.zp + c, ztag, &zc, &pc)) s_ok = 0;
+        if (!get_row(a.zp + c, ztag, a.polls, &zc, &pc)) s_ok = 0;
         return first ? zc : __fmaf_rn(bt, pc, zc);
       };
       float t[R][4];
@@ -451,13 +453,20 @@ __global__ void __launch_bounds__(PV* PT, 1) k_solve(SolveArgs a) {
   }
 #pragma unroll
   for (int i = 0; i < R; ++i)
-    if (row[i] >= 0) a.x[row[i]] = x[i];
+    if (row[i] >= 0) reinterpret_cast<float*>(a.zp + row[i])[0] = x[i];  // (no block reads it after the last exchange)
   if (blockIdx.x == 0 && tid == 0) {
     a.s[S_RZ] = rz;
     a.s[S_RR] = rr;
     a.s[S_BB] = bb;
     a.fail[1] = it;
   }
+}
+
+// x from the rows' words when every wait of the solve was met
+__global__ void __launch_bounds__(PT) k_take(int n, const int* __restrict__ fail, const uint4* __restrict__ zp,
+                                            float* __restrict__ x) {
+  const int i = blockIdx.x * PT + threadIdx.x;
+  if (i < n && !*fail) x[i] = __uint_as_float(zp[i].x);
 }
 
 int grid_blocks(int n) {
@@ -484,9 +493,17 @@ extern "C" size_t fvdbm_pcg_work_bytes(int32_t n) {
 extern "C" int fvdbm_pcg(int32_t n, const int32_t* indptr, const int32_t* indices, const float* values,
                          const float* b, float* x, int32_t max_iter, double rtol, int32_t check_every, void* work,
                          size_t work_bytes, void* stream, int32_t* iters, double* rel_res) {
+  return fvdbm_pcg_bounded(n, indptr, indices, values, b, x, max_iter, rtol, check_every, PCG_POLLS, work, work_bytes,
+                           stream, iters, rel_res);
+}
+
+extern "C" int fvdbm_pcg_bounded(int32_t n, const int32_t* indptr, const int32_t* indices, const float* values,
+                                 const float* b, float* x, int32_t max_iter, double rtol, int32_t check_every,
+                                 int32_t polls, void* work, size_t work_bytes, void* stream, int32_t* iters,
+                                 double* rel_res) {
   if (iters) *iters = 0;
   if (rel_res) *rel_res = 0.0;
-  if (n < 0 || max_iter < 0 || check_every <= 0 || !(rtol >= 0.0)) return FVDBM_EINVAL;
+  if (n < 0 || max_iter < 0 || check_every <= 0 || polls < 0 || polls > PCG_POLLS || !(rtol >= 0.0)) return FVDBM_EINVAL;
   if (n == 0) return FVDBM_OK;
   if (!indptr || !indices || !values || !b || !x || !work || work_bytes < fvdbm_pcg_work_bytes(n))
     return FVDBM_EINVAL;
@@ -524,7 +541,7 @@ extern "C" int fvdbm_pcg(int32_t n, const int32_t* indptr, const int32_t* indice
       if (per_sm * sms >= blocks) {
         // (the exchange words, 96 bytes per 256 rows, fit in one of the five
         // vectors, the rows' words in the four after it)
-        SolveArgs a{n, groups, per_block, max_iter, check_every, rtol, indptr, indices, values, b, x,
+        SolveArgs a{n, groups, per_block, max_iter, check_every, polls, rtol, indptr, indices, values, b, x,
                     reinterpret_cast<uint4*>(r), reinterpret_cast<uint4*>(dinv), s, reinterpret_cast<int*>(s + S_COUNT)};
         void* args[] = {&a};
         struct {
@@ -535,15 +552,19 @@ extern "C" int fvdbm_pcg(int32_t n, const int32_t* indptr, const int32_t* indice
             cudaMemsetAsync(a.ex, 0, size_t(6) * groups * sizeof(uint4), st) != cudaSuccess ||
             cudaMemsetAsync(a.zp, 0, size_t(n) * sizeof(uint4), st) != cudaSuccess ||
             cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), dim3(blocks), dim3(threads), args,
-                                        smem, st) != cudaSuccess ||
+                                        smem, st) != cudaSuccess)
+          return FVDBM_ECUDA;
+        k_take<<<groups, PT, 0, st>>>(n, a.fail, a.zp, x);
+        if (cudaGetLastError() != cudaSuccess ||
             cudaMemcpyAsync(&out, s, sizeof(out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
           return FVDBM_ECUDA;
-        if (out.fail[0]) return FVDBM_EDEVICE;
-        const double bn = out.s[S_BB] > 0.0 ? out.s[S_BB] : 1.0;
-        if (iters) *iters = out.fail[1];
-        if (rel_res) *rel_res = out.s[S_RR] > 0.0 ? std::sqrt(out.s[S_RR] / bn) : 0.0;
-        return FVDBM_OK;
+        if (!out.fail[0]) {
+          const double bn = out.s[S_BB] > 0.0 ? out.s[S_BB] : 1.0;
+          if (iters) *iters = out.fail[1];
+          if (rel_res) *rel_res = out.s[S_RR] > 0.0 ? std::sqrt(out.s[S_RR] / bn) : 0.0;
+          return FVDBM_OK;
+        }
       }
     }
   }

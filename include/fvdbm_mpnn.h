@@ -120,12 +120,18 @@ int fvdbm_mp_to_bf16(const float *x, uint16_t *y, size_t count, void *stream);
  * reproducible.  work: device scratch of at least
  * fvdbm_pcg_work_bytes(n) bytes.  *iters and *rel_res report the end state
  * (rel_res NaN: A was not positive definite or the input not finite).
- * Systems of up to about 300,000 rows run in one cooperative launch;
- * FVDBM_EDEVICE: a bounded wait in it gave up. */
+ * Systems of up to about 300,000 rows run in one cooperative launch whose
+ * waits are bounded; when one runs out the launch-per-kernel form of larger
+ * systems solves the system from the same x (the same bits, later). */
 size_t fvdbm_pcg_work_bytes(int32_t n);
 int fvdbm_pcg(int32_t n, const int32_t *indptr, const int32_t *indices, const float *values, const float *b,
               float *x, int32_t max_iter, double rtol, int32_t check_every, void *work, size_t work_bytes,
               void *stream, int32_t *iters, double *rel_res);
+/* The same with a limit of its own on each wait, in polls (0 .. 2^20, which
+ * fvdbm_pcg takes).  No counterpart in the reference. */
+int fvdbm_pcg_bounded(int32_t n, const int32_t *indptr, const int32_t *indices, const float *values, const float *b,
+                      float *x, int32_t max_iter, double rtol, int32_t check_every, int32_t polls, void *work,
+                      size_t work_bytes, void *stream, int32_t *iters, double *rel_res);
 
 /* Features built on the GPU, one case per call (the host path of
  * fvdbm-jax_gb300/warmstart.py computes the same quantities).  Cell and face
