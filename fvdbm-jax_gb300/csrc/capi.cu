@@ -34,10 +34,11 @@ constexpr double kResidentPart = 0.85, kRingPart = 0.42, kInPlacePart = 0.62;
 // step, per-step kernels / resident: 60k cells 13.0 / 9.9 at 4 steps, 8.2 / 3.2 at 512; 250k 16.9 / 13.8
 // at 4, 12.1 / 6.9 at 64; 300k 16.9 / 16.8 at 4, 14.6 / 12.2 at 8; 400k 17.8 / 20.2
 // at 4, 15.7 / 15.0 at 8, 13.5 / 10.4 at 64; 480k 15.8 / 16.1 at 12, 15.5 / 15.2 at
-// 16, 14.2 / 12.4 at 512.  A launch takes at most kResidentSteps.
+// 16, 14.2 / 12.4 at 512.  A launch takes at most kResidentSteps: it holds every SM, and
+// the steps of other handles wait for it (13 to 50 ms).
 constexpr int kResidentMin = 4, kResidentMinLarge = 8, kResidentMinRing = 16;
 constexpr int kLargeMesh = 1 << 18;  // cells from which AUTO takes the single-launch family
-constexpr int kResidentSteps = 1 << 20;
+constexpr int kResidentSteps = 4096;
 constexpr int kResidentCells = 96;  // cells per block, at least (3.2k cells: 3.4 us per step, 3.9 at 128)
 
 struct Handle {

@@ -6,7 +6,12 @@
 
 namespace fvdbm {
 
-constexpr int RES_POLLS = 1 << 20;  // polls of one import (about a second)
+// Limits of the waits.  A block's neighbour may not have started yet: other streams'
+// kernels may hold the SM that it needs for as long as they run, so an import polls for
+// about ten seconds.  Within a block the cell warps wait for the aux warps, which end an
+// import that gives up: their limit (of tries of up to a microsecond) is the longer one.
+// (Limits by the clock cost registers: 60k cells 3.65 us a step, 3.51 so.)
+constexpr int RES_POLLS = 1 << 24, RES_TRIES = 1 << 28;
 
 // One word of the exchange: three values and a tag, as a single 128-bit access
 // (relaxed, gpu scope: atomic, through L2).
@@ -39,7 +44,7 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar) {
 }
 // Waits for phase `parity` of the barrier, a bounded number of polls.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  for (int it = 0; it < (1 << 24); ++it) {
+  for (int it = 0; it < RES_TRIES; ++it) {
     unsigned done;
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000; selp.u32 %0, 1, 0, p; }"

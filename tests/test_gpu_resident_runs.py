@@ -23,3 +23,58 @@ def test_non_finite_states_far_from_the_walls(runs, flux):
         pdf[((xy - xy.min(0) - span * at) ** 2).sum(1).argmin(), q] = v
     c.pdf = pdf
     _compare(cfn, runs, "auto", "staged")
+
+
+def test_two_handles_side_by_side():
+    """A long run of one handle does not keep the steps of another from running, nor
+    make its blocks give up, and both end as they do alone."""
+    import torch
+
+    from fvdbm_jax_gb300 import Environment
+    cfn = [_case(3200, "upwind"), _case(60_000, "upwind")]
+    alone = []
+    for c in cfn:
+        env = Environment(*c)
+        env.init()
+        env.step(64)
+        alone.append(np.array(env.cells.pdf))
+        env.close()
+    a, b = (Environment(*c) for c in cfn)
+    a.init()
+    b.init()
+    a.step(64)
+    assert np.array_equal(a.cells.pdf, alone[0])
+    a.step(500_000)  # more than a second
+    b.step(64)
+    b.sync()
+    busy = not torch.cuda.ExternalStream(a.stream_ptr).query()
+    assert np.array_equal(b.cells.pdf, alone[1])
+    a.sync()
+    assert busy
+    a.close()
+    b.close()
+
+
+def test_beside_other_kernels():
+    """Runs while another stream keeps the SMs busy."""
+    import torch
+
+    from fvdbm_jax_gb300 import Environment
+    cfn = _case(60_000, "upwind")
+    x = torch.randn((8192, 8192), device="cuda")
+    other = torch.cuda.Stream()
+    got = []
+    for load in (0, 40):
+        env = Environment(*cfn)
+        env.init()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            for _ in range(load):
+                y = x @ x
+        for _ in range(20):
+            env.step(64)
+        env.sync()
+        got.append(np.array(env.cells.pdf))
+        env.close()
+    torch.cuda.synchronize()
+    assert np.array_equal(*got)
