@@ -55,9 +55,13 @@ class Info(C.Structure):
     ]
 
 
+class RunInfo(C.Structure):
+    _fields_ = [("path", C.c_int32), ("blocks", C.c_int32), ("min_steps", C.c_int32), ("readback_beside", C.c_int32)]
+
+
 _LIB = None
 EXPORTS = ["fvdbm_create", "fvdbm_set_state", "fvdbm_step", "fvdbm_step_phase", "fvdbm_get_cells", "fvdbm_get_nodes",
-           "fvdbm_get_face_fluxes", "fvdbm_sync", "fvdbm_stream", "fvdbm_get_info",
+           "fvdbm_get_face_fluxes", "fvdbm_sync", "fvdbm_stream", "fvdbm_get_info", "fvdbm_get_run_info", "fvdbm_run_config",
            "fvdbm_last_error", "fvdbm_destroy", "fvdbm_abi_version", "fvdbm_const_div_check", "fvdbm_const_div_check_form", "fvdbm_wait_selftest",
            "fvdbm_step_static_scratch", "fvdbm_residual", "fvdbm_run_to_steady",
            "fvdbm_batch_create", "fvdbm_batch_config", "fvdbm_batch_residual", "fvdbm_batch_set_active",
@@ -147,6 +151,8 @@ def lib(build_if_missing: bool = True) -> C.CDLL:
     L.fvdbm_stream.argtypes = [vp]
     L.fvdbm_stream.restype = vp
     L.fvdbm_get_info.argtypes = [vp, C.POINTER(Info)]
+    L.fvdbm_get_run_info.argtypes = [vp, C.POINTER(RunInfo)]
+    L.fvdbm_run_config.argtypes = [vp, i32]
     L.fvdbm_last_error.argtypes = [vp]
     L.fvdbm_last_error.restype = C.c_char_p
     L.fvdbm_destroy.argtypes = [vp]

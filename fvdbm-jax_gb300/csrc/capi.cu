@@ -63,7 +63,8 @@ struct Handle {
   int* bar = nullptr;    // its grid-barrier counter
   // resident step (resident.cu): runs of several steps in one launch, with the
   // state on the chip; res_tag: exchange tags used so far
-  bool resident = false;
+  bool resident = false, ring = false;
+  bool on_chip = true;  // fvdbm_run_config
   int res_min = 0;  // steps of a run, at least
   DevResident res{};
   size_t res_ex_bytes = 0;
@@ -285,7 +286,7 @@ constexpr int kPersistSteps = 4096;  // steps per cooperative launch, at most
 // A resident run of n steps may be queued: not a short one, and not while the stream is being captured (the
 // exchange tags of a launch serve once, so it must not be replayed).
 bool resident_ready(Handle* h, int n) {
-  if (!h->resident || n < h->res_min) return false;
+  if (!h->resident || !h->on_chip || n < h->res_min) return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
@@ -496,6 +497,7 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));
   CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
   h->resident = true;
+  h->ring = rp.in_place;
   return FVDBM_OK;
 }
 
@@ -1546,6 +1548,25 @@ int fvdbm_run_to_steady(void* handle, double threshold, int32_t check_every, int
   if (std::isnan(r))
     return fail(h, FVDBM_ENONFINITE, "fvdbm_run_to_steady: the residual turned NaN after " + std::to_string(taken) +
                                          " steps (a cell's rho or u is not finite: the run diverged)");
+  return FVDBM_OK;
+}
+
+int fvdbm_get_run_info(void* handle, fvdbm_run_info_t* info) {
+  if (!handle || !info) return FVDBM_EINVAL;
+  const Handle* h = static_cast<Handle*>(handle);
+  const bool on = h->resident && h->on_chip;
+  info->path = !on ? FVDBM_RUN_LAUNCHES : h->ring ? FVDBM_RUN_RING : FVDBM_RUN_TWO_COPIES;
+  info->blocks = on ? h->res.n_blocks : 0;
+  info->min_steps = on ? h->res_min : 0;
+  info->readback_beside = h->in_ok ? 1 : 0;
+  return FVDBM_OK;
+}
+
+int fvdbm_run_config(void* handle, int32_t on_chip) {
+  if (!handle) return FVDBM_EINVAL;
+  Handle* h = static_cast<Handle*>(handle);
+  if (on_chip != 0 && on_chip != 1) return fail(h, FVDBM_EINVAL, "on_chip must be 0 or 1");
+  h->on_chip = on_chip != 0;
   return FVDBM_OK;
 }
 

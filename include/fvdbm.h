@@ -186,6 +186,23 @@ int fvdbm_set_cells_eq(void *handle, const float *rho, const float *vel);
 /* n_steps applications of Environment.step (src/environment.py:55-65). */
 int fvdbm_step(void *handle, int32_t n_steps);
 
+/* How the handle carries out runs of several steps (no counterpart in the
+ * reference).  fvdbm_run_config: on_chip 0 keeps such runs to the family's
+ * launches, as if the state did not fit; 1 (after creation) gives them back.
+ * The results are the same bits. */
+#define FVDBM_RUN_LAUNCHES 0   /* the family's launches, step by step */
+#define FVDBM_RUN_TWO_COPIES 1 /* one launch, the pdfs on the chip twice */
+#define FVDBM_RUN_RING 2       /* one launch, the pdfs on the chip once */
+typedef struct fvdbm_run_info {
+  int32_t path;             /* FVDBM_RUN_* */
+  int32_t blocks;           /* thread blocks of the one launch, else 0 */
+  int32_t min_steps;        /* shorter runs take the family's launches; 0 with LAUNCHES */
+  int32_t readback_beside;  /* 1: fvdbm_get_cells of rho and vel alone, into page-locked
+                               arrays, would now run beside the last step */
+} fvdbm_run_info_t;
+int fvdbm_get_run_info(void *handle, fvdbm_run_info_t *info);
+int fvdbm_run_config(void *handle, int32_t on_chip);
+
 /* One step split at its kernel boundary so a caller can time each kernel
  * with events on fvdbm_stream(): phase 1 launches the boundary-node kernel
  * (Nodes.calc_pdfs), phase 2 the cell kernel(s) (Faces.calc_fluxes +
