@@ -191,9 +191,10 @@ class Batch:
     def autotune(self, steps: int = 64, candidates=CANDIDATES, use_cache: bool = True) -> dict:
         """Pick the cell kernel's launch shape for this batch's size bucket by
         timing each candidate for ``steps`` steps (the state is saved and
-        restored around the trials).  Decisions are cached per GPU model and
-        size bucket."""
-        key = f"{_device_name(self.device)}|{size_bucket(int(self.cell_ptr[-1]), self.n_cases, self.scheme)}"
+        restored around the trials).  The shape is that of the launches a batch
+        takes when its state does not stay on the chip, so the trials take
+        those.  Decisions are cached per GPU model and size bucket."""
+        key = f"{_device_name(self.device)}|launches|{size_bucket(int(self.cell_ptr[-1]), self.n_cases, self.scheme)}"
         cache = _load_cache() if use_cache else {}
         if key in cache:
             b, w = cache[key]["best"]
@@ -201,12 +202,19 @@ class Batch:
             return cache[key]
         st = self.state()
         times = {}
-        for b, w in candidates:
-            self.config(b, w)
-            self.step(steps // 2).sync()  # warm (graph capture)
-            t0 = time.perf_counter()
-            self.step(steps).sync()
-            times[f"{b}x{w}"] = (time.perf_counter() - t0) / steps
+        run = nat.RunInfo()
+        nat.check(nat.lib().fvdbm_get_run_info(self._h, C.byref(run)), self._h)
+        nat.check(nat.lib().fvdbm_run_config(self._h, 0), self._h)
+        try:
+            for b, w in candidates:
+                self.config(b, w)
+                self.step(steps // 2).sync()  # warm (graph capture)
+                t0 = time.perf_counter()
+                self.step(steps).sync()
+                times[f"{b}x{w}"] = (time.perf_counter() - t0) / steps
+        finally:
+            if run.path != nat.RUN_LAUNCHES:
+                nat.check(nat.lib().fvdbm_run_config(self._h, 1), self._h)
         best = min(times, key=times.get)
         b, w = (int(x) for x in best.split("x"))
         self.config(b, w)

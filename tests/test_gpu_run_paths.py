@@ -136,3 +136,18 @@ def test_batch_by_launches(flux):
             assert np.array_equal(sa[k], sb[k], equal_nan=True), (n, k)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("declined", [False, True])
+def test_autotune_times_the_launches_it_tunes(declined, monkeypatch):
+    from fvdbm_jax_gb300 import Batch
+    b = Batch([_case(n, "upwind", seed=k) for k, n in enumerate((98, 3200))])
+    b.init()
+    if declined:
+        _launches_only(b)
+    seen, step = [], Batch.step
+    monkeypatch.setattr(Batch, "step", lambda self, n=1: (seen.append(_info(self).path), step(self, n))[1])
+    rec = b.autotune(steps=32, use_cache=False)
+    assert set(seen) == {LAUNCHES} and len(seen) == 2 * len(rec["sec_per_step"])
+    assert _info(b).path == (LAUNCHES if declined else TWO_COPIES)
+    b.close()
