@@ -109,7 +109,11 @@ struct Handle {
   cudaStream_t side = nullptr;  // highest priority: its blocks take SM slots as the step's retire
   cudaEvent_t in_ready = nullptr;
   bool in_ok = false;
-  bool stepping = false;  // the last call was fvdbm_step
+  bool stepping = false;  // the stream's last work is a step's: no other call has enqueued any since
+  // single steps since rho and vel were last read back, and how many that read-back
+  // came after: a program that reads back after every so many steps has the last of them
+  // marked, whatever precedes it
+  int singles = 0, read_after = 0;
   int* status_host = nullptr;  // page-locked copy of *status, filled on the stream before a sync
   int* d_rows = nullptr;       // [N] cell indices of a halo pack/unpack
   std::string err;
@@ -254,11 +258,6 @@ int upload_nodes(Handle* h) {
   return FVDBM_OK;
 }
 
-// Steps use programmatic dependent launch between the node and cell kernels
-// (each waits for its predecessor before it reads what one wrote), the first
-// launch of a call when the call before was a step too: single steps, 3.2k
-// cells, 8.0 us, 9.8 without it.  After a copy or another kernel it gains
-// nothing (72 us for state in, step and state out, 74 with it).
 // The plan with the node pointers of buffer a (read) and b (written).
 DevPlan with_nodes(const Handle* h, int a, int b) {
   DevPlan q = h->dp;
@@ -315,7 +314,11 @@ int run_resident(Handle* h, int n) {
   return FVDBM_OK;
 }
 
-// follows: the last work of the stream is a step.
+// Steps use programmatic dependent launch between the node and cell kernels
+// (each waits for its predecessor before it reads what one wrote), the first
+// launch of a call when the stream's last work is a step's (follows): single steps,
+// 3.2k cells, 8.0 us, 9.8 without it.  After a copy or another kernel it gains
+// nothing (72 us for state in, step and state out, 74 with it).
 int enqueue_steps(Handle* h, int n, bool follows = false) {
   if (h->persist && resident_ready(h, n)) return run_resident(h, n);
   if (h->persist) {
@@ -913,7 +916,7 @@ int fvdbm_batch_create(const fvdbm_mesh_t* meshes, const fvdbm_params_t* params,
 int fvdbm_batch_config(void* handle, int32_t block, int32_t prefetch_waves) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   if (!h->batch) return fail(h, FVDBM_EINVAL, "not a batch handle");
   if ((block != 128 && block != 256) || prefetch_waves < 0 || prefetch_waves > 8)
     return fail(h, FVDBM_EINVAL, "block must be 128 or 256 and prefetch_waves 0..8");
@@ -937,6 +940,7 @@ int fvdbm_batch_config(void* handle, int32_t block, int32_t prefetch_waves) {
 static int batch_residual_take(Handle* h, const int32_t* take, double* res_u, double* mass) {
   const HostPlan& hp = h->hp;
   const int S = hp.S;
+  h->stepping = false;
   CK(cudaSetDevice(h->device));
   int rc;
   if (!h->usnap && (rc = dalloc<float>(h, &h->usnap, size_t(2) * hp.Np)) != FVDBM_OK) return rc;
@@ -987,7 +991,7 @@ int fvdbm_batch_residual_cases(void* handle, const int32_t* take, double* res_u,
 int fvdbm_batch_set_active(void* handle, const int32_t* active) {
   if (!handle || !active) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   if (!h->batch) return fail(h, FVDBM_EINVAL, "not a batch handle");
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
@@ -1160,7 +1164,7 @@ static int stage_rows(Handle* h, const int32_t* cells, int32_t n, const void* bu
 int fvdbm_pack_cells(void* handle, const int32_t* cells, int32_t n, float* buf) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   int rc = stage_rows(h, cells, n, buf, "fvdbm_pack_cells");
   if (rc != FVDBM_OK || n == 0) return rc;
   CK(launch_pack_rows(h->f[h->cur], h->d_cell_new, h->d_rows, n, buf, h->stream, h->hp.q));
@@ -1170,7 +1174,7 @@ int fvdbm_pack_cells(void* handle, const int32_t* cells, int32_t n, float* buf) 
 int fvdbm_unpack_cells(void* handle, const int32_t* cells, int32_t n, const float* buf) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   int rc = stage_rows(h, cells, n, buf, "fvdbm_unpack_cells");
   if (rc != FVDBM_OK || n == 0) return rc;
   CK(launch_unpack_rows(h->f[h->cur], h->d_cell_new, h->d_rows, n, buf, h->stream, h->hp.q));
@@ -1211,12 +1215,17 @@ int fvdbm_step(void* handle, int32_t n_steps) {
   if (n_steps < 0) return fail(h, FVDBM_EINVAL, "n_steps < 0");
   CK(cudaSetDevice(h->device));
   h->in_ok = false;
-  // (an event between two steps would part them: only a step that does not
-  // follow another one is marked for the read-back beside it)
-  const bool mark = n_steps == 1 && h->hp.N > 0 && !h->stepping;
+  // An event between two steps parts them (3.2k cells: 9.8 us a step, 8.0 without), so a step
+  // that follows another one is marked only when the read-back is likely to come next, or when
+  // the mesh is so large that it costs nothing.  us per frame of k steps and a read-back,
+  // every step marked / none after the first / this: 250k cells 53.9 / 61.1 / 52.4 at k = 2,
+  // 171 / 159 / 155 at 10; 1M cells 126 / 138 / 126 and 343 / 354 / 342.
+  if (n_steps != 0) h->singles = n_steps == 1 ? h->singles + 1 : 0;
+  const bool mark = n_steps == 1 && h->hp.N > 0 &&
+                    (!h->stepping || h->hp.N >= kLargeMesh || h->singles == h->read_after);
   if (mark) CK(cudaEventRecord(h->in_ready, h->stream));
   const bool follows = h->stepping;
-  h->stepping = true;
+  if (n_steps > 0) h->stepping = true;
   int n = n_steps;
   if (!h->persist && resident_ready(h, n)) {
     int rc = run_resident(h, n);
@@ -1295,7 +1304,7 @@ int fvdbm_const_div_check_form(int32_t device, float divisor, int32_t form, uint
 int fvdbm_step_phase(void* handle, int32_t phase) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   CK(cudaSetDevice(h->device));
   const float* fin = h->f[h->cur];
   float* fout = h->f[h->cur ^ 1];
@@ -1373,6 +1382,10 @@ int fvdbm_get_cells(void* handle, float* pdf, float* rho, float* vel, float* pdf
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
   h->stepping = false;
+  if ((rho || vel) && h->singles > 0) {
+    h->read_after = h->singles;
+    h->singles = 0;
+  }
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   const int N = hp.N;
@@ -1444,6 +1457,7 @@ int fvdbm_get_cells(void* handle, float* pdf, float* rho, float* vel, float* pdf
 int fvdbm_get_nodes(void* handle, float* pdf, float* rho, float* vel) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
+  h->stepping = false;
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   if (hp.M > 0) {
@@ -1470,6 +1484,7 @@ int fvdbm_get_nodes(void* handle, float* pdf, float* rho, float* vel) {
 int fvdbm_get_face_fluxes(void* handle, float* flux) {
   if (!handle || !flux) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
+  h->stepping = false;
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   if (hp.F == 0) return FVDBM_OK;
@@ -1496,6 +1511,7 @@ int fvdbm_residual(void* handle, double* res_u, double* mass) {
   if (!handle || !res_u || !mass) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
   if (h->hp.q != 9) return fail(h, FVDBM_EINVAL, "the convergence monitor supports D2Q9");
+  h->stepping = false;
   const HostPlan& hp = h->hp;
   CK(cudaSetDevice(h->device));
   const int nb = residual_chunks(hp.N, kResidualChunk);
@@ -1678,7 +1694,7 @@ int scratch_address(Handle* h, float** out) {
 extern "C" int fvdbm_step_static_scratch(void* handle, int32_t n_steps) {
   if (!handle) return FVDBM_EINVAL;
   Handle* h = static_cast<Handle*>(handle);
-  h->in_ok = false;
+  h->in_ok = h->stepping = false;
   const HostPlan& hp = h->hp;
   if (n_steps < 0) return fail(h, FVDBM_EINVAL, "n_steps < 0");
   if (h->fused || h->tile || h->one || h->batch)

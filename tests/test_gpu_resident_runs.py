@@ -78,3 +78,57 @@ def test_beside_other_kernels():
         env.close()
     torch.cuda.synchronize()
     assert np.array_equal(*got)
+
+
+def _beside(env):
+    from test_gpu_run_paths import _info
+    return bool(_info(env).readback_beside)
+
+
+@pytest.mark.parametrize("cells", [3200, 270_000])
+def test_which_single_steps_are_read_back_beside(cells):
+    """rho and vel of the step's input, read while the step runs: after a step that
+    follows other work, after the last of as many steps as the frame before had, and on
+    large meshes after any; the values are those of a read-back that waits."""
+    import torch
+
+    from fvdbm_jax_gb300 import Environment
+    from fvdbm_jax_gb300 import _native as nat
+    L, large = nat.lib(), cells >= 1 << 18
+    cfn = _case(cells, "upwind")
+    env, ref = Environment(*cfn), Environment(*cfn, kernel="staged")
+    env.init()
+    ref.init()
+    h = env.handle
+    N = np.shape(cfn[0].pdf)[0]
+    rho, vel = (torch.zeros(s).pin_memory().numpy() for s in ((N,), (N, 2)))
+    rows = np.arange(4, dtype=np.int32)
+    buf = torch.zeros((4, 9), device="cuda")
+
+    def step(k, beside):
+        for _ in range(k):
+            env.step()
+            ref.step()
+        assert _beside(env) == beside
+
+    def read():
+        nat.check(L.fvdbm_get_cells(h, None, nat.fptr(rho), nat.fptr(vel), None), h)
+        assert np.array_equal(rho, np.asarray(ref.cells.rho).reshape(-1))
+        assert np.array_equal(vel, ref.cells.vel)
+
+    for first, k in ((True, 1), (True, 1), (large, 3), (True, 3), (True, 3)):
+        step(k, first)
+        read()
+    step(1, True)
+    step(1, large)
+    pack = lambda: nat.check(L.fvdbm_pack_cells(h, nat.iptr(rows), 4, buf.data_ptr()), h)
+    unpack = lambda: nat.check(L.fvdbm_unpack_cells(h, nat.iptr(rows), 4, buf.data_ptr()), h)
+    for other in (pack, lambda: (pack(), unpack()), env.residual, lambda: env.nodes.pdf):
+        other()
+        step(1, True)
+        read()
+    env.step(0)
+    step(1, True)
+    read()
+    env.close()
+    ref.close()
