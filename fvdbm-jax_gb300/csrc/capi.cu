@@ -443,22 +443,18 @@ std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh, co
     return rp;
   };
   try {
-    return std::async(std::launch::async, plan);
-  } catch (const std::system_error&) {  // no thread to be had: planned when it is asked for
-    return std::async(std::launch::deferred, plan);
+    try {
+      return std::async(std::launch::async, plan);
+    } catch (const std::system_error&) {  // no thread to be had: planned when it is asked for
+      return std::async(std::launch::deferred, plan);
+    }
+  } catch (const std::bad_alloc&) {
+    return {};
   }
 }
 
-int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
-  if (!plan.valid()) return FVDBM_OK;
+int upload_resident(Handle* h, const ResidentPlan& rp) {
   const HostPlan& hp = h->hp;
-  ResidentPlan rp;
-  try {
-    rp = plan.get();
-  } catch (const std::bad_alloc&) {
-    return fail(h, FVDBM_ENOMEM, "host memory for the resident step's tables");
-  }
-  if (!rp.ok) return FVDBM_OK;
   DevResident& r = h->res;
   bool fits = false;
   CK(rp.in_place ? prepare_in_place(h->dp, rp, r, &fits) : prepare_resident(h->dp, rp, r, &fits));
@@ -493,6 +489,11 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   const size_t rows_at = ex_at + (h->res_ex_bytes + 255) / 256 * 256;
   unsigned char* base = nullptr;
   int rc = dalloc(h, &base, rows_at + size_t(12) * rp.n_rows * sizeof(float), &buf);
+  if (rc == FVDBM_ENOMEM) {
+    cudaGetLastError();
+    h->err.clear();
+    return FVDBM_OK;
+  }
   if (rc != FVDBM_OK) return rc;
   for (auto& a : at) *a.first = base + a.second;
   r.ex = reinterpret_cast<uint4*>(base + ex_at);
@@ -502,6 +503,18 @@ int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
   h->resident = true;
   h->ring = rp.in_place;
   return FVDBM_OK;
+}
+
+// The tables are not necessary: without the memory for them, on the host or the
+// device, runs take the family's launches.
+int make_resident(Handle* h, std::future<ResidentPlan>& plan) {
+  if (!plan.valid()) return FVDBM_OK;
+  try {
+    const ResidentPlan rp = plan.get();
+    return rp.ok ? upload_resident(h, rp) : FVDBM_OK;
+  } catch (const std::bad_alloc&) {
+    return FVDBM_OK;
+  }
 }
 
 // Cell blocks (of the batch launch's block size) holding cells of active

@@ -151,3 +151,36 @@ def test_autotune_times_the_launches_it_tunes(declined, monkeypatch):
     assert set(seen) == {LAUNCHES} and len(seen) == 2 * len(rec["sec_per_step"])
     assert _info(b).path == (LAUNCHES if declined else TWO_COPIES)
     b.close()
+
+
+def test_creation_without_memory_for_the_tables():
+    """A handle whose launches fit in the device's memory and whose tables of the run on the
+    chip do not: it is created, and its runs take the launches."""
+    import torch
+
+    from fvdbm_jax_gb300 import Environment
+    cfn = _case(400_000, "lax_wendroff")
+    need, got = [], []
+    for kernel in ("fused_nodes", "auto"):  # without and with the tables
+        env = Environment(*cfn, kernel=kernel)
+        env.init()
+        env.step(9)
+        got.append(np.array(env.cells.pdf))
+        need.append(env.info()["device_bytes"])
+        env.close()
+    tables = need[1] - need[0]
+    assert tables > 30e6
+    torch.cuda.empty_cache()
+    ballast = torch.empty(int(torch.cuda.mem_get_info()[0] - need[0] - tables / 2), dtype=torch.uint8, device="cuda")
+    env = Environment(*cfn)
+    try:
+        env.init()
+        env.step(9)
+        got.append(np.array(env.cells.pdf))
+        path = _info(env).path
+    finally:
+        env.close()
+        del ballast
+        torch.cuda.empty_cache()
+    assert path == LAUNCHES
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
