@@ -97,6 +97,7 @@ struct Handle {
   float* nbuf[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
   int node_cur = 0, node_last = 1;
   bool nodes_ready = false;
+  bool own_capture = false;  // get_graph is capturing
   // convergence monitor (fvdbm_residual)
   float* usnap = nullptr;   // [2][Np] velocity at the previous residual call
   double* red = nullptr;    // chunk partials, then the 4 totals
@@ -270,13 +271,21 @@ DevPlan with_nodes(const Handle* h, int a, int b) {
   return q;
 }
 
+bool capturing(const Handle* h) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
 // In-kernel node update: the boundary nodes of the next step, computed once
-// from the recorded stencil macros after an upload (the step kernels then
-// keep them current).
+// from the recorded stencil macros after an upload or a run on the chip (the step
+// kernels then keep them current).  A graph that the caller captures computes
+// them itself: what comes between its replays may leave them to the next step.
 int ensure_nodes(Handle* h) {
-  if (!h->fnodes || h->nodes_ready) return FVDBM_OK;
+  if (!h->fnodes) return FVDBM_OK;
+  const bool graph = !h->own_capture && capturing(h);
+  if (h->nodes_ready && !graph) return FVDBM_OK;
   CK(launch_nodes_cp(with_nodes(h, h->node_cur, h->node_cur), h->f[h->cur], h->stream, false));
-  h->nodes_ready = true;
+  if (!graph) h->nodes_ready = true;
   return FVDBM_OK;
 }
 
@@ -285,9 +294,7 @@ constexpr int kPersistSteps = 4096;  // steps per cooperative launch, at most
 // A resident run of n steps may be queued: not a short one, and not while the stream is being captured (the
 // exchange tags of a launch serve once, so it must not be replayed).
 bool resident_ready(Handle* h, int n) {
-  if (!h->resident || !h->on_chip || n < h->res_min) return false;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  return h->resident && h->on_chip && n >= h->res_min && !capturing(h);
 }
 
 // n steps in resident launches.  Afterwards the handle is as after n single
@@ -299,14 +306,15 @@ int run_resident(Handle* h, int n) {
       CK(cudaMemsetAsync(h->res.ex, 0, h->res_ex_bytes, h->stream));
       h->res_tag = 0;
     }
-    const DevPlan p = h->fnodes ? with_nodes(h, h->node_cur, h->node_cur) : h->dp;
-    const int last = h->cur ^ (k & 1);
+    // (the nodes of the last step in the buffer that single steps leave them in)
+    const int nodes = h->node_cur ^ (k & 1) ^ 1, last = h->cur ^ (k & 1);
+    const DevPlan p = h->fnodes ? with_nodes(h, nodes, nodes) : h->dp;
     CK(launch_resident(p, h->res, h->f[h->cur], h->f[last ^ 1], h->f[last], k, h->res_tag, h->stream));
     h->res_tag += unsigned(k);
     h->cur = last;
     if (h->fnodes) {
-      h->node_last = h->node_cur;
-      h->node_cur ^= 1;
+      h->node_last = nodes;
+      h->node_cur = nodes ^ 1;
       h->nodes_ready = false;
     }
     n -= k;
@@ -403,7 +411,9 @@ int get_graph(Handle* h, int parity, cudaGraphExec_t* out) {
   const int save = h->cur, save_nc = h->node_cur, save_nl = h->node_last;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  h->own_capture = true;
   int rc = enqueue_steps(h, kGraphSteps);
+  h->own_capture = false;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   h->cur = save;
   h->node_cur = save_nc;

@@ -132,3 +132,47 @@ def test_which_single_steps_are_read_back_beside(cells):
     read()
     env.close()
     ref.close()
+
+
+@pytest.mark.parametrize("cells,kernel", [(3200, "auto"), (3200, "fast"), (270_000, "auto")])
+def test_replays_of_a_captured_graph_between_runs(cells, kernel):
+    """Steps captured by the caller (which are launches, whatever their number) go on from
+    the state that runs, single steps and setters leave, and the other way round."""
+    import torch
+
+    from fvdbm_jax_gb300 import Environment
+    cfn = _case(cells, "upwind")
+    a, b = (Environment(*cfn, kernel=kernel) for _ in range(2))
+    a.init()
+    b.init()
+    a.step(2)
+    a.sync()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(a.stream_ptr), capture_error_mode="thread_local"):
+        a.step(20)
+    done = 2
+
+    def replay():
+        with torch.cuda.stream(torch.cuda.ExternalStream(a.stream_ptr)):
+            g.replay()
+
+    for n, graph in ((0, True), (16, True), (2, True), (17, False), (1, True), (20, False), (6, True), (0, True)):
+        a.step(n)
+        done += n
+        if graph:
+            replay()
+            done += 20
+    a.sync()
+    for _ in range(done):
+        b.step()
+    assert np.array_equal(a.cells.pdf, b.cells.pdf)
+    pdf = np.array(cfn[0].pdf)
+    a.cells.pdf = pdf
+    b.cells.pdf = pdf
+    replay()
+    a.step(16)
+    for _ in range(36):
+        b.step()
+    assert np.array_equal(a.cells.pdf, b.cells.pdf)
+    a.close()
+    b.close()
