@@ -912,6 +912,8 @@ def predict_cases(net, cases, rho_in, rho_out, batch_cells: int = 2_000_000, rto
             bins = torch.empty(ng, dtype=torch.int32, device=dev)
             count = torch.zeros(nb * len(grp), dtype=torch.int32, device=dev)
             for j, (k, go) in enumerate(zip(grp, gofs[:-1])):
+                if not arr[k]["N"]:
+                    raise ValueError("a case without cells has no bins")
                 lo, hi = arr[k]["lo"], arr[k]["hi"]
                 sp = np.maximum(hi - lo, 1e-30)
                 chk(L.fvdbm_ws_bin_ids(arr[k]["N"], P(D[k]["cen"]), float(lo[0]), float(lo[1]), float(sp[0]),
