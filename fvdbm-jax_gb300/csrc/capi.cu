@@ -469,14 +469,17 @@ int upload_resident(Handle* h, const ResidentPlan& rp) {
   bool fits = false;
   CK(rp.in_place ? prepare_in_place(h->dp, rp, r, &fits) : prepare_resident(h->dp, rp, r, &fits));
   if (!fits) return FVDBM_OK;
-  // one allocation for all, one copy for the tables
-  std::vector<unsigned char> buf;
-  std::vector<std::pair<const void**, size_t>> at;  // field, offset
+  // one allocation for all; one copy for the small tables, and the large ones from
+  // where they are
+  constexpr size_t kLarge = size_t(1) << 18;
+  struct Part {
+    const void** field;
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Part> parts;
   auto put = [&](auto& field, const auto& vec) {
-    const size_t o = (buf.size() + 255) / 256 * 256, n = vec.size() * sizeof(vec[0]);
-    buf.resize(o + std::max<size_t>(n, 16));
-    if (n) std::memcpy(buf.data() + o, vec.data(), n);
-    at.push_back({reinterpret_cast<const void**>(&field), o});
+    parts.push_back({reinterpret_cast<const void**>(&field), vec.data(), vec.size() * sizeof(vec[0]), 0});
   };
   put(r.block, rp.block);
   put(r.dev, rp.dev);
@@ -494,7 +497,17 @@ int upload_resident(Handle* h, const ResidentPlan& rp) {
   put(r.en_w, rp.en_w);
   put(r.fz_dev, rp.fz_dev);
   put(r.gh, rp.gh);
-  const size_t ex_at = (buf.size() + 255) / 256 * 256;
+  size_t ex_at = 0;
+  std::vector<unsigned char> buf;
+  for (int large = 0; large < 2; ++large)
+    for (Part& q : parts) {
+      if ((q.bytes >= kLarge) != (large == 1)) continue;
+      q.at = ex_at;
+      ex_at += (std::max<size_t>(q.bytes, 16) + 255) / 256 * 256;
+      if (large) continue;
+      buf.resize(ex_at);
+      if (q.bytes) std::memcpy(buf.data() + q.at, q.src, q.bytes);
+    }
   h->res_ex_bytes = size_t(2) * ((hp.q + 2) / 3) * size_t(std::max(rp.n_export, 1)) * sizeof(uint4);
   const size_t rows_at = ex_at + (h->res_ex_bytes + 255) / 256 * 256;
   unsigned char* base = nullptr;
@@ -505,7 +518,10 @@ int upload_resident(Handle* h, const ResidentPlan& rp) {
     return FVDBM_OK;
   }
   if (rc != FVDBM_OK) return rc;
-  for (auto& a : at) *a.first = base + a.second;
+  for (const Part& q : parts) {
+    *q.field = base + q.at;
+    if (q.bytes >= kLarge) CK(cudaMemcpyAsync(base + q.at, q.src, q.bytes, cudaMemcpyHostToDevice, h->stream));
+  }
   r.ex = reinterpret_cast<uint4*>(base + ex_at);
   r.rows = reinterpret_cast<float*>(base + rows_at);
   CK(cudaMemsetAsync(r.ex, 0, h->res_ex_bytes, h->stream));

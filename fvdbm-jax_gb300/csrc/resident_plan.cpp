@@ -15,7 +15,9 @@ namespace fvdbm {
 
 namespace {
 
-constexpr int MANY = 1 << 16;  // cells from which threads pay
+// Cells from which threads pay.  ms of a plan on 16 host cores, one thread / these: 10k cells
+// 1.3 / 1.0, 20k 2.5 / 1.4, 60k 6.3 / 2.4, 250k 20.0 (most of it on one) / 8.7.
+constexpr int MANY = 1 << 14;
 
 struct Point {
   float x[2];
@@ -62,19 +64,17 @@ int chunk_cells(int inner, int threads) {
   return std::max(32, ((inner + n - 1) / n + 31) / 32 * 32);
 }
 
-// f(t) of every block, by a few threads for a large mesh of N cells (by fewer, or
-// the caller, when there are none to be had).
-template <class F>
-void for_blocks(int N, int B, const F& f) {
-  if (N < MANY) {
-    for (int t = 0; t < B; ++t) f(t);
-    return;
-  }
-  constexpr int THREADS = 8;
-  std::vector<std::future<void>> work;
+// f(t, scratch) of every block, by a few threads for a large mesh of N cells (by fewer, or
+// the caller, when there are none to be had), each with its own make().
+template <class M, class F>
+void for_blocks(int N, int B, const M& make, const F& f) {
+  const int THREADS = N < MANY ? 1 : 8;
   auto run = [&](int i) {
-    for (int t = i; t < B; t += THREADS) f(t);
+    auto scratch = make();
+    for (int t = i; t < B; t += THREADS) f(t, scratch);
   };
+  if (THREADS == 1) return run(0);
+  std::vector<std::future<void>> work;
   for (int i = 0; i < THREADS && i < B; ++i) {
     try {
       work.push_back(std::async(std::launch::async, run, i));
@@ -84,6 +84,19 @@ void for_blocks(int N, int B, const F& f) {
   }
   for (auto& w : work) w.get();
 }
+template <class F>
+void for_blocks(int N, int B, const F& f) {
+  for_blocks(N, B, [] { return 0; }, [&](int t, int) { f(t); });
+}
+
+// Tables of one block, before they are joined: indices into themselves.
+struct BlockTables {
+  std::vector<int32_t> halo_dev, halo_exp, st_loc, halo_st, nd, fz_dev, gh;
+  std::vector<uint32_t> en_st;
+  std::vector<float> nd_sw, en_w;
+  bool usable = true;
+  int rows = 0, stride = 0;
+};
 
 // Order of the update in place: the interior cells, the first `inner` of the
 // part's n, along the longer side of its bounding box, in chunks of TC.  Within
@@ -122,9 +135,18 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     std::memcpy(&x, &u, 4);
     return x;
   };
-  for (size_t g = 0; g < hp.hf.size() / (size_t(H) * 32); ++g)
-    for (size_t i = 3 * 32; i < size_t(H) * 32; ++i)
-      if (!std::isfinite(f32(hp.hf[g * H * 32 + i]))) return;
+  const int G = int(hp.hf.size() / (size_t(H) * 32)), share_of = 256;  // groups of 32 cells, by 256
+  std::vector<char> finite((G + share_of - 1) / share_of, 1);
+  for_blocks(N, int(finite.size()), [&](int t) {
+    uint32_t most = 0;  // (all exponent bits set: not finite)
+    for (int g = t * share_of; g < std::min(G, (t + 1) * share_of); ++g) {
+      const uint32_t* w = hp.hf.data() + size_t(g) * H * 32;
+      for (int i = 3 * 32; i < H * 32; ++i) most = std::max(most, w[i] & 0x7f800000u);
+    }
+    finite[t] = most != 0x7f800000u;
+  });
+  for (char ok : finite)
+    if (!ok) return;
   for (float a : hp.inv_area)
     if (!std::isfinite(a)) return;
   const bool lw = hp.scheme == FVDBM_LAX_WENDROFF, sc = hp.variant == FVDBM_VARIANT_FACE_SCALE;
@@ -173,22 +195,17 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   // face reads belongs to the block of its first stencil cell.
   std::vector<std::vector<int32_t>> imp(B), nodes(B);
   std::vector<std::vector<int32_t>> ghost_cells(B);
-  std::vector<int32_t> mark(N, -1), nmark(hp.M, -1);
   std::vector<char> node_used(hp.M, 0);
-  for (int c = 0; c < N; ++c)
-    for (int k = 0; k < 3; ++k) {
-      const int32_t code = int32_t(hp.hf[hfi(c, k)]);
-      if (code & HF_GHOST) node_used[hp.gh_a[code >> HF_SHIFT]] = node_used[hp.gh_b[code >> HF_SHIFT]] = 1;
-    }
+  for (size_t g = 0; g < hp.gh_a.size(); ++g) node_used[hp.gh_a[g]] = node_used[hp.gh_b[g]] = 1;
   std::vector<std::vector<int32_t>> extra(B);
   for (int d = 0; d < hp.Mc; ++d)
     if (!node_used[d])
       extra[hp.nd_ptr[d + 1] > hp.nd_ptr[d] ? part[hp.nd_cell[hp.nd_ptr[d]] & ~ND_NEQ_ZERO] : 0].push_back(d);
   std::vector<char> links(size_t(B) * B, 0);  // links[t * B + u]: t imports from u
-  for (int t = 0; t < B; ++t) {
+  const auto no_node = [&] { return std::vector<int32_t>(hp.M, -1); };
+  for_blocks(N, B, no_node, [&](int t, std::vector<int32_t>& nmark) {
     auto need = [&](int32_t c) {
-      if (part[c] != t && mark[c] != t) {
-        mark[c] = t;
+      if (part[c] != t) {
         imp[t].push_back(c);
         links[size_t(t) * B + part[c]] = 1;
       }
@@ -212,7 +229,9 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
         }
       }
     for (int32_t d : extra[t]) node(d);
-  }
+    std::sort(imp[t].begin(), imp[t].end());
+    imp[t].erase(std::unique(imp[t].begin(), imp[t].end()), imp[t].end());
+  });
   // a block may overwrite an exported value only once its reader has moved
   // on, which it learns from the reader's own exports: every link goes both
   // ways (a one-way link gets one cell to read back)
@@ -234,20 +253,20 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   // (an exported cell waits for the imports too: its next value overwrites
   // the one that its readers must have taken)
   std::vector<char> kind(exported);
-  for (int c = 0; c < N; ++c)
-    for (int k = 0; k < 3; ++k) {
-      const int32_t code = int32_t(hp.hf[hfi(c, k)]);
-      if (code & HF_GHOST)
-        kind[c] = 2;
-      else if (part[code >> HF_SHIFT] != part[c])
-        kind[c] = std::max<char>(kind[c], 1);
-    }
   for (int t = 0; t < B; ++t) rp.max_own = std::max(rp.max_own, part_end[t] - (t ? part_end[t - 1] : 0));
   if (!in_place) resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
   std::vector<int> inside(B);  // interior cells
   for_blocks(N, B, [&](int t) {
     const auto first = ids.begin() + (t ? part_end[t - 1] : 0), last = ids.begin() + part_end[t];
     std::sort(first, last);
+    for (auto c = first; c != last; ++c)
+      for (int k = 0; k < 3; ++k) {
+        const int32_t code = int32_t(hp.hf[hfi(*c, k)]);
+        if (code & HF_GHOST)
+          kind[*c] = 2;
+        else if (part[code >> HF_SHIFT] != t)
+          kind[*c] = std::max<char>(kind[*c], 1);
+      }
     const auto in_end = std::stable_partition(first, last, [&](int32_t c) { return kind[c] == 0; });
     std::stable_partition(in_end, last, [&](int32_t c) { return kind[c] == 1; });
     inside[t] = int(in_end - first);
@@ -281,8 +300,10 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     rp.block.push_back(mb);
   }
   rp.dev.assign(off, -1);
-  rp.exp.assign(off, -1);
-  rp.cls.assign(off / 32, 0);
+  if (!in_place) {  // (the ring has its classes in its order, and the slots in its codes)
+    rp.exp.assign(off, -1);
+    rp.cls.assign(off / 32, 0);
+  }
   rp.hf.assign(size_t(off / 32) * R * 32, 0u);
   auto ri = [&](int i, int row) { return size_t(i >> 5) * size_t(R) * 32 + size_t(row) * 32 + (i & 31); };
   auto bits = [](float x) {
@@ -292,36 +313,41 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   };
   const HfRows HR{3, hp.scheme, hp.variant};
   if (hp.fv) rp.inv_area.assign(off, 0.0f);
-  std::vector<int32_t> hloc(N, -1), nloc(hp.M, -1), sloc(N, -1);
-  std::vector<char> node_owned(hp.M, 0);
-  bool usable = true;
-  for (int t = 0; t < B; ++t) {
+  std::vector<int32_t> owner(hp.M, -1);  // the first block that computes the node
+  for (int t = 0; t < B; ++t)
+    for (int32_t d : nodes[t])
+      if (owner[d] < 0) owner[d] = t;
+  struct Scratch {
+    std::vector<int32_t> hloc, nloc, sloc;
+  };
+  const auto scratch = [&] {
+    return Scratch{std::vector<int32_t>(N), std::vector<int32_t>(hp.M), std::vector<int32_t>(N, -1)};
+  };
+  std::vector<BlockTables> tables(B);
+  for_blocks(N, B, scratch, [&](int t, Scratch& sc_) {
+    auto& [hloc, nloc, sloc] = sc_;
     ResidentBlock& mb = rp.block[t];
+    BlockTables& bt = tables[t];
     const int a = t ? part_end[t - 1] : 0, pad = (mb.nown + 31) / 32 * 32;
     const int bnd0 = (mb.nin + 31) / 32 * 32, nb = mb.nown - mb.nin;
     std::sort(imp[t].begin(), imp[t].end(), [&](int32_t x, int32_t y) { return slot[x] < slot[y]; });
-    mb.halo_off = int(rp.halo_dev.size());
     mb.nhalo = int(imp[t].size());
     const int halo0 = in_place ? 0 : pad;
     for (int j = 0; j < mb.nhalo; ++j) {
-      rp.halo_dev.push_back(imp[t][j]);
-      rp.halo_exp.push_back(slot[imp[t][j]]);
+      bt.halo_dev.push_back(imp[t][j]);
+      bt.halo_exp.push_back(slot[imp[t][j]]);
       hloc[imp[t][j]] = halo0 + j;
     }
     auto local = [&](int32_t c) { return part[c] == t ? loc[c] : hloc[c]; };
     // boundary nodes: computed first, then frozen
     std::stable_partition(nodes[t].begin(), nodes[t].end(), [&](int32_t d) { return d < hp.Mc; });
-    mb.nd_off = int(rp.nd.size() / 4);
-    mb.fz_off = int(rp.fz_dev.size());
-    mb.st_off = int(rp.st_loc.size());
     mb.last_st = 0;
-    mb.en_off = int(rp.en_st.size());
     std::vector<int32_t> touched;
     // (in place: the block's own ones first)
     auto st = [&](int32_t c) {
       if (sloc[c] < 0) {
         sloc[c] = mb.nst++;
-        rp.st_loc.push_back(local(c));
+        bt.st_loc.push_back(local(c));
         touched.push_back(c);
       }
       return sloc[c];
@@ -341,31 +367,29 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       const int32_t d = nodes[t][j];
       nloc[d] = int(j);
       if (d >= hp.Mc) {
-        rp.fz_dev.push_back(d);
+        bt.fz_dev.push_back(d);
         ++mb.nf;
         continue;
       }
       ++mb.nn;
       if (hp.nd_npad[d] > 0) mb.last_st = st(hp.last_cell_new);
-      rp.nd.push_back(d);
-      rp.nd.push_back(hp.nd_type[d] | (hp.nd_npad[d] > 0 ? 4 : 0) | (node_owned[d] ? 0 : 8));
-      rp.nd.push_back(int(rp.en_st.size()));
-      rp.nd.push_back(hp.nd_ptr[d + 1] - hp.nd_ptr[d]);
-      rp.nd_sw.push_back(hp.nd_sumw[d]);
-      node_owned[d] = 1;
+      bt.nd.push_back(d);
+      bt.nd.push_back(hp.nd_type[d] | (hp.nd_npad[d] > 0 ? 4 : 0) | (owner[d] == t ? 8 : 0));
+      bt.nd.push_back(int(bt.en_st.size()));
+      bt.nd.push_back(hp.nd_ptr[d + 1] - hp.nd_ptr[d]);
+      bt.nd_sw.push_back(hp.nd_sumw[d]);
       for (int e = hp.nd_ptr[d]; e < hp.nd_ptr[d + 1]; ++e) {
         const uint32_t code = hp.nd_cell[e];
-        rp.en_st.push_back(uint32_t(st(int32_t(code & ~ND_NEQ_ZERO))) | (code & ND_NEQ_ZERO));
-        rp.en_w.push_back(hp.nd_w[e]);
+        bt.en_st.push_back(uint32_t(st(int32_t(code & ~ND_NEQ_ZERO))) | (code & ND_NEQ_ZERO));
+        bt.en_w.push_back(hp.nd_w[e]);
       }
     }
-    for (int j = 0; in_place && j < mb.nhalo; ++j) rp.halo_st.push_back(sloc[imp[t][j]]);
+    for (int j = 0; in_place && j < mb.nhalo; ++j) bt.halo_st.push_back(sloc[imp[t][j]]);
     for (int32_t c : touched) sloc[c] = -1;
-    mb.ne = int(rp.en_st.size()) - mb.en_off;
+    mb.ne = int(bt.en_st.size());
     // face slots with local indices; ghost faces get their own entries.  In
     // place: the boundary cells' name rows, those of interior neighbours (saved)
     // and of boundary cells after the ghosts
-    mb.gh_off = int(rp.gh.size() / 4);
     int ng = 0;
     for (int i = 0; in_place && i < mb.nown; ++i)
       for (int k = 0; k < 3; ++k) {
@@ -381,15 +405,17 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       }
     const int orow = mb.nhalo + ng, brow = orow + mb.nsave, ring = bnd0 + mb.chunk;
     // (16 bits for a neighbour, 12 for a link)
-    if (in_place && (std::max(brow + nb, 9 * (ring + nb + 31)) > 0xffff || std::max(mb.nsave, nb) >= 0xfff)) usable = false;
+    if (in_place && (std::max(brow + nb, 9 * (ring + nb + 31)) > 0xffff || std::max(mb.nsave, nb) >= 0xfff)) bt.usable = false;
     for (int i = 0; i < mb.nown; ++i) {
       const int32_t c = ids[a + i];
       const int l = loc[c], g = mb.own_off + l;
       const bool inside = i < mb.nin;
       rp.dev[g] = c;
-      rp.exp[g] = slot[c];
       if (hp.fv) rp.inv_area[g] = hp.inv_area[c];
-      rp.cls[g / 32] = std::max<int32_t>(rp.cls[g / 32], kind[c]);
+      if (!in_place) {
+        rp.exp[g] = slot[c];
+        rp.cls[g / 32] = std::max<int32_t>(rp.cls[g / 32], kind[c]);
+      }
       for (int row = 3; row < (hp.fast ? H : 12); ++row) rp.hf[ri(g, row)] = hp.hf[hfi(c, row)];
       if (!hp.fast)
         for (int k = 0; k < 3; ++k) {
@@ -402,7 +428,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
             const float v[6] = {nx, ny, nx + ny, ny - nx, 2.0f * nx, 2.0f * ny};
             for (int j = 0; j < NP; ++j) {
               const float t = (v[j] * (case_dt ? case_dt[mb.cs] : pr.delta_t)) / D2;
-              if (!std::isfinite(t)) usable = false;
+              if (!std::isfinite(t)) bt.usable = false;
               rp.hf[ri(g, 15 + 3 * j + k)] = bits(t);
             }
           }
@@ -417,13 +443,13 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
           std::memcpy(&rbits, &hp.gh_r[gi], 4);
           idx = (in_place ? mb.nhalo : pad + mb.nhalo) + mb.ng++;
           const int32_t row4[4] = {l, nloc[hp.gh_a[gi]], nloc[hp.gh_b[gi]], rbits};
-          rp.gh.insert(rp.gh.end(), row4, row4 + 4);
+          bt.gh.insert(bt.gh.end(), row4, row4 + 4);
         } else {
           const int32_t n = code >> HF_SHIFT;
           idx = local(n);
           if (inside) {
             // the sweep overwrites a chunk once the next one has been read
-            if (idx < mb.nin && std::abs(idx / mb.chunk - l / mb.chunk) > 1) usable = false;
+            if (idx < mb.nin && std::abs(idx / mb.chunk - l / mb.chunk) > 1) bt.usable = false;
             idx = idx < mb.nin ? idx : ring + idx - bnd0;  // (the boundary cells follow the ring)
             idx = (idx >> 5) * 288 + (idx & 31);
           } else if (in_place && part[n] == t) {
@@ -435,9 +461,36 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
         rp.hf[ri(g, k)] = uint32_t((code & HF_SLOT1) | (idx << HF_SHIFT)) | link << IP_LINK;
       }
     }
+    bt.rows = orow + 2 * (mb.nsave + nb);
+    bt.stride = in_place ? bnd0 + mb.chunk + 2 * ((nb + 31) / 32 * 32) : pad + mb.nhalo + mb.ng;
+  });
+  // ---- the blocks' tables one after the other
+  bool usable = true;
+  auto join = [](auto& all, const auto& own) { all.insert(all.end(), own.begin(), own.end()); };
+  for (int t = 0; t < B; ++t) {
+    ResidentBlock& mb = rp.block[t];
+    BlockTables& bt = tables[t];
+    usable = usable && bt.usable;
+    mb.halo_off = int(rp.halo_dev.size());
+    mb.nd_off = int(rp.nd.size() / 4);
+    mb.fz_off = int(rp.fz_dev.size());
+    mb.st_off = int(rp.st_loc.size());
+    mb.en_off = int(rp.en_st.size());
+    mb.gh_off = int(rp.gh.size() / 4);
     mb.row_off = rp.n_rows;
-    rp.n_rows += orow + 2 * (mb.nsave + nb);
-    rp.stride = std::max(rp.stride, in_place ? bnd0 + mb.chunk + 2 * ((nb + 31) / 32 * 32) : pad + mb.nhalo + mb.ng);
+    for (size_t j = 2; j < bt.nd.size(); j += 4) bt.nd[j] += mb.en_off;
+    join(rp.halo_dev, bt.halo_dev);
+    join(rp.halo_exp, bt.halo_exp);
+    join(rp.st_loc, bt.st_loc);
+    join(rp.halo_st, bt.halo_st);
+    join(rp.nd, bt.nd);
+    join(rp.nd_sw, bt.nd_sw);
+    join(rp.en_st, bt.en_st);
+    join(rp.en_w, bt.en_w);
+    join(rp.fz_dev, bt.fz_dev);
+    join(rp.gh, bt.gh);
+    rp.n_rows += bt.rows;
+    rp.stride = std::max(rp.stride, bt.stride);
     rp.max_nodes = std::max(rp.max_nodes, mb.nn + mb.nf);
     rp.max_st = std::max(rp.max_st, mb.nst);
     rp.max_table = std::max(rp.max_table, 8 * mb.nn + 4 * mb.ng + 2 * mb.ne + mb.nst + 2 * mb.nhalo);
