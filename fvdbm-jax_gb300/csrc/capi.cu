@@ -26,17 +26,31 @@ constexpr int kGraphSteps = 32;  // steps per captured graph (even)
 // (the rest: halos, tables), or D2Q9 upwind through a ring (resident_in_place.cu)
 // up to a part that leaves room for the ring's free chunk and the
 // boundary cells.  The ring's two halves of a block's warps work side by side, but
-// wait for each other once a step; us per step, two copies / ring (porous):
-// 130k cells 4.9 / 5.4, 180k 5.5 / 5.6, 250k 7.7 / 6.6, 320k 8.9 / 7.5; contracted
-// family 180k 4.7 / 5.3, 250k 6.7 / 6.1.
+// wait for each other once a step.  us per step in runs of 512, porous meshes, two copies /
+// ring: 129k cells 4.95 / 5.58, 179k 5.55 / 5.64, 204k 5.88 / 6.18, 249k 7.92 / 6.56, 318k
+// 8.87 / 7.47; contracted family 179k 4.78 / 5.34, 249k 6.70 / 6.01.
 constexpr double kResidentPart = 0.85, kRingPart = 0.42, kInPlacePart = 0.62;
-// The steps of a run, at least: a launch loads and stores the whole state.  us per
-// step, per-step kernels / resident: 60k cells 13.0 / 9.9 at 4 steps, 8.2 / 3.2 at 512; 250k 16.9 / 13.8
-// at 4, 12.1 / 6.9 at 64; 300k 16.9 / 16.8 at 4, 14.6 / 12.2 at 8; 400k 17.8 / 20.2
-// at 4, 15.7 / 15.0 at 8, 13.5 / 10.4 at 64; 480k 15.8 / 16.1 at 12, 15.5 / 15.2 at
-// 16, 14.2 / 12.4 at 512.  A launch takes at most kResidentSteps: it holds every SM, and
+// The steps of a run, at least: a launch loads and stores the whole state, and the per-step
+// launches gain on the ring as meshes grow.  us per step, per-step launches / on the chip:
+//   two copies  3.2k cells, runs of 4: 7.6 / 4.7; 60k channel 4: 8.8 / 5.1; Lax-Wendroff, cavity,
+//               255k 4: 16.4 / 9.8, contracted 11.4 / 10.2; 400k 8: 14.3 / 13.0, contracted 11.2 / 11.2
+//   ring        (cavities, the meshes whose launches are the fastest) 255k 4: 11.5 / 8.8,
+//               contracted 4: 9.1 / 9.8, 6: 9.0 / 8.5; 330k 8: 10.8 / 9.7; 400k 8: 11.1 / 11.3,
+//               12: 11.1 / 10.3 (porous 395k 8: 13.7 / 13.1); 425k finite volume 12: 10.8 / 11.0, 16: 10.8 / 10.5; 520k 16:
+//               11.9 / 12.2, 24: 11.9 / 11.7; 600k 24: 12.8 / 13.2, 48: 12.7 / 12.6
+// (porous, contracted, 468k 16: 11.7 / 11.8, 64: 11.6 / 10.6).  A batch's launches are slower (24
+// cases, 253k cells 4: 14.0 / 11.3; 423k 16: 17.5 / 12.4), and the one cooperative launch of
+// FVDBM_KERNEL_PERSIST costs as much as a resident one (249k cells, one step: 22.6 / 18.8;
+// 395k 25.6 / 27.5, two 22.7 / 19.6).  twice: two copies would fit.
+int run_min(int N, bool ring, bool fast, bool persist, bool batch, bool twice) {
+  if (persist) return !twice ? 16 : ring && N >= 350000 ? 2 : 1;
+  if (N < 1 << 18) return ring && fast ? 6 : 4;
+  if (batch) return twice ? 8 : 16;
+  if (!ring || N < 350000) return 8;
+  return N < 410000 ? 10 : N < 450000 ? 16 : N < 500000 ? 18 : N < 540000 ? 24 : 48;
+}
+// A launch takes at most kResidentSteps: it holds every SM, and
 // the steps of other handles wait for it (13 to 50 ms).
-constexpr int kResidentMin = 4, kResidentMinLarge = 8, kResidentMinRing = 16;
 constexpr int kLargeMesh = 1 << 18;  // cells from which AUTO takes the single-launch family
 constexpr int kResidentSteps = 4096;
 constexpr int kResidentCells = 96;  // cells per block, at least (3.2k cells: 3.4 us per step, 3.9 at 128)
@@ -63,7 +77,7 @@ struct Handle {
   int* bar = nullptr;    // its grid-barrier counter
   // resident step (resident.cu): runs of several steps in one launch, with the
   // state on the chip; res_tag: exchange tags used so far
-  bool resident = false, ring = false;
+  bool resident = false, ring = false, res_twice = false;
   bool on_chip = true;  // fvdbm_run_config
   int res_min = 0;  // steps of a run, at least
   DevResident res{};
@@ -439,12 +453,10 @@ std::future<ResidentPlan> start_resident(Handle* h, const fvdbm_mesh_t& mesh, co
       cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess || hp.N == 0)
     return {};
   const double chip = double(sms) * lim;
-  const bool twice = double(hp.N) * 2 * hp.q * 4 <= kResidentPart * chip;
+  const bool twice = h->res_twice = double(hp.N) * 2 * hp.q * 4 <= kResidentPart * chip;
   const bool ring = hp.q == 9 && hp.scheme == FVDBM_UPWIND && hp.variant == 0 &&
                     double(hp.N) * 2 * hp.q * 4 > kRingPart * chip && double(hp.N) * hp.q * 4 <= kInPlacePart * chip;
   if (!twice && !ring) return {};
-  // (the one cooperative launch of FVDBM_KERNEL_PERSIST costs as much)
-  h->res_min = !twice ? kResidentMinRing : h->persist ? 1 : hp.N < kLargeMesh ? kResidentMin : kResidentMinLarge;
   const int blocks = std::min(sms, (hp.N + kResidentCells - 1) / kResidentCells);
   auto plan = [h, &mesh, blocks, case_dt, twice, ring] {
     ResidentPlan rp;
@@ -528,6 +540,7 @@ int upload_resident(Handle* h, const ResidentPlan& rp) {
   CK(cudaStreamSynchronize(h->stream));  // the tables' copies have left the host vectors
   h->resident = true;
   h->ring = rp.in_place;
+  h->res_min = run_min(hp.N, h->ring, hp.fast, h->persist, h->batch, h->res_twice);
   return FVDBM_OK;
 }
 

@@ -64,7 +64,7 @@ extern "C" {
                                      FUSED below and for D2Q13, STAGED when the fused kernels
                                      cannot run: not triangles, padded or foreign face slots,
                                      per-q flux scale).  Runs of several steps (fvdbm_step with
-                                     n_steps >= 4, 8 or 16 by size) of a mesh whose state fits on
+                                     n_steps >= 4 to 48 by size) of a mesh whose state fits on
                                      the chip (D2Q9 about 400,000 triangles, upwind about 600,000)
                                      take one launch, with the same results; FAST and packed
                                      batches do too */

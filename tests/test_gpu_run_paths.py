@@ -31,10 +31,12 @@ def _launches_only(env):
     (98, "upwind", "D2Q9", "fast", TWO_COPIES, 4), (3200, "upwind", "D2Q9", "persist", TWO_COPIES, 1),
     (96_000, "upwind", "D2Q9", "auto", TWO_COPIES, 4), (96_000, "lax_wendroff", "D2Q13", "auto", TWO_COPIES, 4),
     (120_000, "lax_wendroff", "D2Q9", "fast", TWO_COPIES, 4), (215_000, "upwind", "D2Q9", "auto", RING, 4),
-    (270_000, "upwind", "D2Q9", "auto", RING, 8), (300_000, "upwind", "D2Q9", "fast", RING, 8),
+    (240_000, "upwind", "D2Q9", "fast", RING, 6), (270_000, "upwind", "D2Q9", "auto", RING, 8),
+    (300_000, "upwind", "D2Q9", "fast", RING, 8), (320_000, "upwind", "D2Q9", "persist", RING, 1),
+    (400_000, "upwind", "D2Q9", "persist", RING, 2), (400_000, "upwind", "D2Q9", "auto", RING, 10),
     (400_000, "lax_wendroff", "D2Q9", "auto", TWO_COPIES, 8), (270_000, "upwind", "D2Q13", "auto", TWO_COPIES, 8),
     (420_000, "upwind", "D2Q9", "auto", RING, 16), (430_000, "upwind", "D2Q9", "persist", RING, 16),
-    (600_000, "upwind", "D2Q9", "auto", RING, 16),
+    (490_000, "upwind", "D2Q9", "auto", RING, 18), (520_000, "upwind", "D2Q9", "fast", RING, 24), (600_000, "upwind", "D2Q9", "auto", RING, 48),
     (450_000, "lax_wendroff", "D2Q9", "auto", LAUNCHES, 0), (650_000, "upwind", "D2Q9", "auto", LAUNCHES, 0),
     (3200, "upwind", "D2Q9", "fused", LAUNCHES, 0), (3200, "upwind", "D2Q9", "fused_nodes", LAUNCHES, 0),
     (3200, "upwind", "D2Q9", "staged", LAUNCHES, 0), (3200, "upwind", "D2Q13", "staged", LAUNCHES, 0)])
@@ -89,6 +91,12 @@ def test_runs_by_launches(cells, mesh, special, lattice, flux, kernel):
         _same(a, b, (kernel, n))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("cells,kernel,runs", [(400_000, "auto", (9, 10, 1, 17)), (520_000, "fast", (23, 24, 1, 31)),
+                                               (600_000, "auto", (47, 48, 1, 53))])
+def test_shortest_runs_of_the_ring(cells, kernel, runs):
+    _compare(_case(cells, "upwind"), runs, kernel, "fast" if kernel == "fast" else "fused")
 
 
 def test_persistent_runs_beyond_the_chip():
