@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "../../include/fvdbm_mpnn.h"
 
@@ -370,7 +371,14 @@ __global__ void k_spmm(const int* __restrict__ row_ptr, const int* __restrict__ 
   *o = accumulate ? *o + s : s;
 }
 
-constexpr int LONG_ROW = 8;  // chunks from which a row is summed by a block
+// Chunks from which a row is summed by a block (k_spmm_long_rows, 4 us and 8 ns a chunk) and
+// no longer by a thread per feature (33 ns a chunk), when such rows are launched for at all: the
+// mean row is that long, or there are so many chunks that the launch does not show (some of
+// them may be one row's).  us by threads / by blocks, width 64: 1 row of 64 chunks 9.3 / 10.4,
+// 157 12.4 / 12.4, 7,813 270 / 73; 16 rows of 50 10.4 / 10.4, 196 16.5 / 12.4; 256 rows of 31 12.4 / 14.4,
+// 100 18.6 / 20.6.  Widths that are no multiple of LRF lose at every size (32: 264 / 281).
+constexpr int LONG_ROW = 128, MANY_CHUNKS = 1 << 18;
+constexpr int LRC = 128, LRF = 64;  // chunks per stage, features per block
 
 // Long rows in chunks: pass 1 folds each chunk's entries (at most a few
 // dozen, in order) per feature into partial[chunk][f]; pass 2 folds a row's
@@ -387,10 +395,10 @@ __global__ void k_spmm_chunks(const int* __restrict__ chunk_start, const int* __
 }
 
 __global__ void k_spmm_rows(const int* __restrict__ chunk_ptr, int n, const float* __restrict__ partial, int d,
-                            float* __restrict__ out, int accumulate) {
+                            float* __restrict__ out, int accumulate, int long_row) {
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int i = int(t / d), f = int(t % d);
-  if (i >= n || chunk_ptr[i + 1] - chunk_ptr[i] >= LONG_ROW) return;
+  if (i >= n || chunk_ptr[i + 1] - chunk_ptr[i] >= long_row) return;
   float s = 0.0f;
   for (int c = chunk_ptr[i]; c < chunk_ptr[i + 1]; ++c) s += partial[size_t(c) * d + f];
   float* o = out + size_t(i) * d + f;
@@ -400,10 +408,7 @@ __global__ void k_spmm_rows(const int* __restrict__ chunk_ptr, int n, const floa
 // The same fold, same order, for rows of at least LONG_ROW chunks: a block per
 // row brings its partials to shared memory, 128 chunks ahead of one warp per 32
 // features that adds them in order from there: the serial chain is one add per
-// chunk.  (One thread per row and feature waited for each load: 530 us for the
-// 7,800 chunks of a 500k-cell mean, this 20.)  A block first looks for the long
-// rows of its share of the rows.
-constexpr int LRC = 128, LRF = 64;  // chunks per stage, features per block
+// chunk.  A block first looks for the long rows of its share of the rows.
 __global__ void __launch_bounds__(512) k_spmm_long_rows(const int* __restrict__ chunk_ptr, int n,
                                                         const float* __restrict__ partial, int d,
                                                         float* __restrict__ out, int accumulate) {
@@ -623,8 +628,10 @@ int fvdbm_mp_spmm_chunked(const int32_t* chunk_start, const int32_t* chunk_ptr, 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (nchunks > 0)
     k_spmm_chunks<<<nblk(size_t(nchunks) * d, 256), 256, 0, s>>>(chunk_start, col, wt, nchunks, h, d, partial);
-  k_spmm_rows<<<nblk(size_t(n) * d, 256), 256, 0, s>>>(chunk_ptr, n, partial, d, out, accumulate);
-  if (nchunks >= LONG_ROW) {
+  const bool by_blocks = d % LRF == 0 && (nchunks / LONG_ROW >= n || nchunks >= MANY_CHUNKS);
+  k_spmm_rows<<<nblk(size_t(n) * d, 256), 256, 0, s>>>(chunk_ptr, n, partial, d, out, accumulate,
+                                                     by_blocks ? LONG_ROW : INT_MAX);
+  if (by_blocks) {
     constexpr int smem = 2 * LRC * LRF * 4;
     if (cudaFuncSetAttribute(k_spmm_long_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
     k_spmm_long_rows<<<dim3(std::min(n, 4 * sm_count()), (d + LRF - 1) / LRF), 512, smem, s>>>(chunk_ptr, n, partial, d,
