@@ -28,7 +28,8 @@ constexpr int kGraphSteps = 32;  // steps per captured graph (even)
 // boundary cells.  The ring's two halves of a block's warps work side by side, but
 // wait for each other once a step.  us per step in runs of 512, porous meshes, two copies /
 // ring: 129k cells 4.95 / 5.58, 179k 5.55 / 5.64, 204k 5.88 / 6.18, 249k 7.92 / 6.56, 318k
-// 8.87 / 7.47; contracted family 179k 4.78 / 5.34, 249k 6.70 / 6.01.
+// 8.87 / 7.47; contracted family 179k 4.78 / 5.34, 249k 6.70 / 6.01 (cavities, whose parts have fewer
+// boundary cells: 205k 4.9 / 6.0 in runs of 64, 251k 5.64 / 5.94, 400k 8.68 / 8.48).
 constexpr double kResidentPart = 0.85, kRingPart = 0.42, kInPlacePart = 0.62;
 // The steps of a run, at least: a launch loads and stores the whole state, and the per-step
 // launches gain on the ring as meshes grow.  us per step, per-step launches / on the chip:

@@ -18,7 +18,7 @@
 // rest is below an ulp.  Products are issued from the smallest piece up.  The weight
 // gradient's accumulator is drained every tile and summed in FP32 registers:
 // the tensor core truncates where it adds, and a chain over a block's thousands of
-// cells would drift (each tile's is 48 long).
+// cells would drift (each tile's is 24 long: six pairs of pieces by four steps of 16 cells).
 //
 // Operand tiles are [rows][64] bfloat16 in the 128-byte swizzle (row r's 16-byte
 // chunk c at chunk c ^ (r & 7)).  Read along the rows' 64 entries they are the

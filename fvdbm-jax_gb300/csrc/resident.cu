@@ -21,13 +21,13 @@
 // What bounds it: on small meshes (up to ~400 cells per block) the chain
 // import, stencil macros, nodes, ghosts, boundary cells, export of the blocks at the
 // boundary, about 6,500 clocks; beyond, the cell warps' issue and shared-memory
-// slots.  us per step, best per-step family before / now (runs of 512
-// steps): 3.2k cells 7.2 / 3.1, 60k upwind 8.2 / 3.2, 60k Lax-Wendroff 10.2 /
-// 3.4, 60k D2Q13 14.2 / 4.9, 250k 10.9 / 7.6, 400k 10.7 / 7.9 (D2Q9 upwind takes
-// resident_in_place.cu from 206k on).  One barrier for
-// all warps and the nodes in line with the cells measured 3.4, 4.5, 5.7, 6.8,
-// 10.4 and 11.5; row-wise tables read through L1 each step 3.3, 3.3, 3.5, 4.9, 8.4
-// and 8.7.
+// slots.  us per step in runs of 512, per-step launches / here: cavity 3.2k cells 7.3 / 3.3;
+// channel with cylinder, 60k, upwind 8.2 / 3.2, Lax-Wendroff 9.9 / 3.4, D2Q13 12.9 / 4.9; porous
+// 129k 10.7 / 5.0, 179k 10.5 / 5.6, Lax-Wendroff 204k 14.0 / 6.6, 328k 14.5 / 10.1, D2Q13 179k
+// 17.0 / 8.4 (D2Q9 upwind takes resident_in_place.cu from 206k on; two copies there: porous 249k
+// 7.9, cavity 251k 5.6).  Tried on meshes of 3.2k to 400k cells: one
+// barrier for all warps and the nodes in line with the cells took 1.1 to 1.7 times as
+// long, row-wise tables read through L1 each step 1.0 to 1.1 times.
 //
 // The states are bit for bit those of the same number of single steps: every
 // sum and product is that of fvdbm_cell.cuh and d2q13.cuh, element by element.

@@ -18,10 +18,11 @@
 //
 // Bound by latency, at 425k cells: the sweep takes about 3,200 clocks per chunk of 512
 // cells (525 instructions per cell on 16 warps), the aux warps' chain of rounds
-// through the halo import about 18,000; both run at once.  us per step, one or two
-// launches of a step / here: porous, 250k cells 12.1 / 6.6, 425k 13.6 / 9.9, contracted
-// family 11.1 / 6.1 and 11.4 / 8.7; 24 cases of 422k cells in all 22 / 15.  Boundary
-// cells after the sweep, by the cell warps: 11.1 and 8.8 at 425k.
+// through the halo import about 18,000; both run at once.  us per step in runs of 512,
+// one or two launches of a step / here: porous, 249k cells 12.1 / 6.6, 420k 13.7 / 9.9, contracted
+// family 10.6 / 6.0 and 11.6 / 8.7; cavity, 425k 10.8 / 9.1, contracted 9.2 / 7.2; 24 cases of
+// 423k cells in all 17.1 / 11.2.  Boundary cells after the sweep, by the cell warps: porous,
+// 420k 11.1 and 8.8.
 #include "resident.cuh"
 
 namespace fvdbm {
@@ -492,8 +493,9 @@ InPlaceKern pick_in_place(const DevPlan& p) {
 // Threads of a block: the cell warps, then the aux warps.  A chunk takes about as
 // long with fewer cell threads (latency) and a round of the aux warps 2-4
 // thousand clocks, so half of the threads each; 576 to the cells where that saves
-// the largest block a chunk.  us per step (exact, fast; porous, 425k cells): 12.7,
-// 11.3 with 768 cell threads, 11.5, 10.1 with 640, 10.3, 8.3 with 512.
+// the largest block a chunk.  us per step (exact, fast; porous, 420k cells): 12.3,
+// 11.8 with 768 cell threads, 11.4, 11.1 with 640, 9.9, 8.7 with 576, 10.0, 8.7 with 512, 11.3,
+// 8.7 with 384.
 void in_place_threads(int max_in, int* cell_threads, int* threads) {
   *cell_threads = (max_in + 575) / 576 < (max_in + 511) / 512 ? 576 : 512;
   *threads = IP_THREADS;
