@@ -15,9 +15,11 @@ namespace fvdbm {
 
 namespace {
 
-// Cells from which threads pay.  ms of a plan on 16 host cores, one thread / these: 10k cells
-// 1.3 / 1.0, 20k 2.5 / 1.4, 60k 6.3 / 2.4, 250k 20.0 (most of it on one) / 8.7.
-constexpr int MANY = 1 << 14;
+// Threads for a mesh of N cells: one for every so many, the caller among them.  ms of a plan on 16
+// host cores, one thread / these: 12k cells 1.7 / 1.0, 20k 2.5 / 1.3, 60k 6.3 / 2.3, 250k 20.0 (most
+// of it on one) / 8.7; a thread for every 1,500 or 6,000 cells 1.0 and 1.4 at 12k.
+constexpr int THREAD_CELLS = 3000, THREADS = 8;
+int threads_for(int N) { return std::max(1, std::min(THREADS, N / THREAD_CELLS)); }
 
 struct Point {
   float x[2];
@@ -27,7 +29,8 @@ struct Point {
 // Recursive bisection of pts[a, b) (device cells) into parts [p0, p0 + parts)
 // of equal size, each cut across the longer side of its bounding box: compact
 // parts keep the halos short.  Without coordinates the device order is cut.
-void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, std::vector<int32_t>& part_end) {
+void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, std::vector<int32_t>& part_end,
+            int many) {
   if (parts == 1) {
     part_end[p0] = b;
     return;
@@ -48,14 +51,15 @@ void bisect(bool xy, std::vector<Point>& pts, int a, int b, int p0, int parts, s
   }
   std::future<void> other;  // (a large part's halves side by side)
   try {
-    if (b - a > MANY) other = std::async(std::launch::async, [&] { bisect(xy, pts, a, mid, p0, left, part_end); });
+    if (b - a > many)
+      other = std::async(std::launch::async, [&] { bisect(xy, pts, a, mid, p0, left, part_end, many); });
   } catch (const std::system_error&) {
   }
-  bisect(xy, pts, mid, b, p0 + left, parts - left, part_end);
+  bisect(xy, pts, mid, b, p0 + left, parts - left, part_end, many);
   if (other.valid())
     other.get();
   else
-    bisect(xy, pts, a, mid, p0, left, part_end);
+    bisect(xy, pts, a, mid, p0, left, part_end, many);
 }
 
 // Cells of a chunk of the sweep: chunks of equal size, at most a cell per thread.
@@ -64,24 +68,24 @@ int chunk_cells(int inner, int threads) {
   return std::max(32, ((inner + n - 1) / n + 31) / 32 * 32);
 }
 
-// f(t, scratch) of every block, by a few threads for a large mesh of N cells (by fewer, or
-// the caller, when there are none to be had), each with its own make().
+// f(t, scratch) of every block, by a few threads (by fewer when there are none to be
+// had), each with its own make().
 template <class M, class F>
 void for_blocks(int N, int B, const M& make, const F& f) {
-  const int THREADS = N < MANY ? 1 : 8;
+  const int n = threads_for(N);
   auto run = [&](int i) {
     auto scratch = make();
-    for (int t = i; t < B; t += THREADS) f(t, scratch);
+    for (int t = i; t < B; t += n) f(t, scratch);
   };
-  if (THREADS == 1) return run(0);
   std::vector<std::future<void>> work;
-  for (int i = 0; i < THREADS && i < B; ++i) {
+  for (int i = 1; i < n && i < B; ++i) {
     try {
       work.push_back(std::async(std::launch::async, run, i));
     } catch (const std::system_error&) {
       run(i);
     }
   }
+  run(0);
   for (auto& w : work) w.get();
 }
 template <class F>
@@ -184,7 +188,8 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       pts[i] = Point{{xy ? xy[2 * size_t(c)] : 0.0f, xy ? xy[2 * size_t(c) + 1] : 0.0f}, i};
     }
     for (int s = 0, p0 = 0; s < S; p0 += share[s++])
-      bisect(xy != nullptr, pts, case_cell[s], case_cell[s + 1], p0, share[s], part_end);
+      bisect(xy != nullptr, pts, case_cell[s], case_cell[s + 1], p0, share[s], part_end,
+             std::max(THREAD_CELLS, N / THREADS));
     for (int i = 0; i < N; ++i) ids[i] = pts[i].id;
   }
   for (int t = 0, i = 0; t < B; ++t)
