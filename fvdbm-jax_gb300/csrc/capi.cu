@@ -1627,7 +1627,7 @@ int fvdbm_get_run_info(void* handle, fvdbm_run_info_t* info) {
   info->path = !on ? FVDBM_RUN_LAUNCHES : h->ring ? FVDBM_RUN_RING : FVDBM_RUN_TWO_COPIES;
   info->blocks = on ? h->res.n_blocks : 0;
   info->min_steps = on ? h->res_min : 0;
-  info->readback_beside = h->in_ok ? 1 : 0;
+  info->readback_beside = h->in_ok && h->hp.q == 9 ? 1 : 0;
   return FVDBM_OK;
 }
 

@@ -16,7 +16,7 @@ namespace fvdbm {
 namespace {
 
 // Threads for a mesh of N cells: one for every so many, the caller among them.  ms of a plan on 16
-// host cores, one thread / these: 12k cells 1.7 / 1.0, 20k 2.5 / 1.3, 60k 6.3 / 2.3, 250k 20.0 (most
+// host cores, one thread / these: 12k cells 1.7 / 0.9, 20k 2.5 / 1.3, 60k 6.3 / 2.3, 250k 20.0 (most
 // of it on one) / 8.7; a thread for every 1,500 or 6,000 cells 1.0 and 1.4 at 12k.
 constexpr int THREAD_CELLS = 3000, THREADS = 8;
 int threads_for(int N) { return std::max(1, std::min(THREADS, N / THREAD_CELLS)); }
@@ -100,6 +100,13 @@ struct BlockTables {
   std::vector<float> nd_sw, en_w;
   bool usable = true;
   int rows = 0, stride = 0;
+  void clear() {
+    for (auto* v : {&halo_dev, &halo_exp, &st_loc, &halo_st, &nd, &fz_dev, &gh}) v->clear();
+    en_st.clear();
+    nd_sw.clear();
+    en_w.clear();
+    usable = true;
+  }
 };
 
 // Order of the update in place: the interior cells, the first `inner` of the
@@ -260,10 +267,14 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
   std::vector<char> kind(exported);
   for (int t = 0; t < B; ++t) rp.max_own = std::max(rp.max_own, part_end[t] - (t ? part_end[t - 1] : 0));
   if (!in_place) resident_threads(rp.max_own, &rp.cell_threads, &rp.threads);
+  {  // each part's cells in device order
+    std::vector<int32_t> at(B, 0);
+    for (int t = 1; t < B; ++t) at[t] = part_end[t - 1];
+    for (int i = 0; i < N; ++i) ids[at[part[i]]++] = i;
+  }
   std::vector<int> inside(B);  // interior cells
   for_blocks(N, B, [&](int t) {
     const auto first = ids.begin() + (t ? part_end[t - 1] : 0), last = ids.begin() + part_end[t];
-    std::sort(first, last);
     for (auto c = first; c != last; ++c)
       for (int k = 0; k < 3; ++k) {
         const int32_t code = int32_t(hp.hf[hfi(*c, k)]);
@@ -324,15 +335,16 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
       if (owner[d] < 0) owner[d] = t;
   struct Scratch {
     std::vector<int32_t> hloc, nloc, sloc;
+    BlockTables bt;  // (grown once, copied for each block)
   };
   const auto scratch = [&] {
-    return Scratch{std::vector<int32_t>(N), std::vector<int32_t>(hp.M), std::vector<int32_t>(N, -1)};
+    return Scratch{std::vector<int32_t>(N), std::vector<int32_t>(hp.M), std::vector<int32_t>(N, -1), {}};
   };
   std::vector<BlockTables> tables(B);
   for_blocks(N, B, scratch, [&](int t, Scratch& sc_) {
-    auto& [hloc, nloc, sloc] = sc_;
+    auto& [hloc, nloc, sloc, bt] = sc_;
     ResidentBlock& mb = rp.block[t];
-    BlockTables& bt = tables[t];
+    bt.clear();
     const int a = t ? part_end[t - 1] : 0, pad = (mb.nown + 31) / 32 * 32;
     const int bnd0 = (mb.nin + 31) / 32 * 32, nb = mb.nown - mb.nin;
     std::sort(imp[t].begin(), imp[t].end(), [&](int32_t x, int32_t y) { return slot[x] < slot[y]; });
@@ -468,6 +480,7 @@ void build_resident(const fvdbm_mesh_t& m, const fvdbm_params_t& pr, const HostP
     }
     bt.rows = orow + 2 * (mb.nsave + nb);
     bt.stride = in_place ? bnd0 + mb.chunk + 2 * ((nb + 31) / 32 * 32) : pad + mb.nhalo + mb.ng;
+    tables[t] = bt;
   });
   // ---- the blocks' tables one after the other
   bool usable = true;
